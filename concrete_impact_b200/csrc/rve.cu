@@ -1,12 +1,10 @@
 // Periodic structured Hex8 RVE kernels (sm_100a): fused residual, deterministic periodic
-// gather, matrix-free PCG, homogenisation.
+// gather, homogenisation (the PCG solve is in rve_pcg.cu).
 //
 // Restates, for structured periodic boxes, the reference's
 //   _compute_hex8_strain_fields + material update + _assemble_force_and_tangent
 //       (src/fem/assembly/nonlinear_solid.py:428-493) -- fused into rve_residual_kernel;
 //   u = T w + A ebar and r = T^T f_int (src/fem/rve/solver.py:88-100, periodic.py:20-169);
-//   the reduced solve K_red dw = -r (solver.py:143-144), done here by Jacobi-PCG with a
-//       matrix-free tangent apply instead of SuperLU;
 //   the homogenisation and diagnostics of _build_rve_response (solver.py:253-364);
 //   the Schur-complement effective tangent (solver.py:438-461) via multi-RHS PCG.
 //
@@ -25,13 +23,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <cooperative_groups.h>
-
 #include "cib_common.cuh"
 #include "j2vp_point.cuh"
 #include "rve.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace cib {
 
@@ -65,35 +59,6 @@ __device__ __forceinline__ void physical_grads(int q, const RveDesc& d, Grad8<T>
     G.x[a] = e8x * fy[ay] * fz[az] * sx;
     G.y[a] = e8y * fx[ax] * fz[az] * sy;
     G.z[a] = e8z * fx[ax] * fy[ay] * sz;
-  }
-}
-
-// The gradients of all 8 Gauss points of a box element in shared memory, entry (a, d) of
-// point q at tab[(3 a + d) * 8 + q]: the lanes of a warp that share q read the same word.
-// The PCG kernels fill it once per solve (one RVE per system; a thread's Gauss point is
-// fixed because the item stride is a multiple of 8) instead of forming the gradients for
-// every element of every CG iteration.
-template <typename T>
-__device__ __forceinline__ void fill_grad_table(const RveDesc& d, T* tab) {
-  if (threadIdx.x < 8) {
-    Grad8<T> G;
-    physical_grads((int)threadIdx.x, d, G);
-#pragma unroll
-    for (int a = 0; a < 8; ++a) {
-      tab[(3 * a + 0) * 8 + threadIdx.x] = G.x[a];
-      tab[(3 * a + 1) * 8 + threadIdx.x] = G.y[a];
-      tab[(3 * a + 2) * 8 + threadIdx.x] = G.z[a];
-    }
-  }
-}
-
-template <typename T>
-__device__ __forceinline__ void load_grads(const T* tab, int q, Grad8<T>& G) {
-#pragma unroll
-  for (int a = 0; a < 8; ++a) {
-    G.x[a] = tab[(3 * a + 0) * 8 + q];
-    G.y[a] = tab[(3 * a + 1) * 8 + q];
-    G.z[a] = tab[(3 * a + 2) * 8 + q];
   }
 }
 
@@ -527,504 +492,6 @@ __global__ void __launch_bounds__(RVE_THREADS) rve_gather_norms_kernel(const Rve
 }
 
 // ---------------------------------------------------------------------------------------
-// One element-Gauss-point item of the matrix-free apply and its loads.  The apply loops
-// fetch the next round's item (the vector values at its node, its phase and tangent flag,
-// then its tangent parameters) while the current round computes, so that the L2 latency of
-// those loads overlaps the arithmetic instead of stalling every round.
-template <typename T>
-struct ApplyItem {
-  bool live;
-  int el, q, ph, flag;
-  int64_t g;
-  T mine[3];
-  T tp[8];
-};
-
-template <typename T>
-__device__ __forceinline__ void fetch_item(const RvePcgArgs<T>& a, const RveDesc& d, const double* __restrict__ p,
-                                           int items, int nxy, int k, int it, ApplyItem<T>& x) {
-  const int gl = it * blockDim.x + threadIdx.x;
-  x.live = gl < items;
-  x.el = x.live ? (gl >> 3) : 0;
-  x.q = gl & 7;
-  const int j = x.el / d.nx, i = x.el - j * d.nx;
-  const int64_t e = d.eoff + x.el + (int64_t)nxy * k;
-  x.g = 8 * e + x.q;
-  x.ph = 0;
-  x.flag = 0;
-#pragma unroll
-  for (int dd = 0; dd < 3; ++dd) x.mine[dd] = (T)0;
-  if (x.live) {
-    const int64_t node = element_node(d, i, j, k, x.q);
-#pragma unroll
-    for (int dd = 0; dd < 3; ++dd) x.mine[dd] = (T)__ldcg(p + 3 * node + dd);  // other ranks may have written p
-    x.ph = (int)a.phase[e];
-    x.flag = (int)a.tflag[x.g];
-  }
-}
-
-template <typename T>
-__device__ __forceinline__ void fetch_tangent(const RvePcgArgs<T>& a, ApplyItem<T>& x) {
-  if (x.live && x.flag) {
-#pragma unroll
-    for (int c = 0; c < 8; ++c) x.tp[c] = a.tparam[c * a.ngp + x.g];
-  }
-}
-
-// Element-node contributions w B^T C B u of one item (valid on every lane; zero when the
-// item is not live), reduce-scattered so that lane q holds node q's three values.
-template <typename T>
-__device__ __forceinline__ void apply_item(const RvePcgArgs<T>& a, const ApplyItem<T>& x, const T* gtab, T jw,
-                                           T out[3]) {
-  T u[8][3];
-  allgather8(x.mine, u);
-  Grad8<T> Gr;
-  load_grads(gtab, x.q, Gr);
-  T eps[6], sig[6];
-  strain_from(Gr, u, eps);
-  TangentParams<T> tp;
-  tp.elastic = 1;
-  tp.f = (T)0;
-  tp.c = (T)0;
-#pragma unroll
-  for (int c = 0; c < 6; ++c) tp.n[c] = (T)0;
-  if (x.live && x.flag) {
-    tp.elastic = 0;
-#pragma unroll
-    for (int c = 0; c < 6; ++c) tp.n[c] = x.tp[c];
-    tp.f = x.tp[6];
-    tp.c = x.tp[7];
-  }
-  tangent_apply(a.mats.m[x.ph], tp, eps, sig);
-  T f[8][3];
-  bt_stress(Gr, sig, x.live ? jw : (T)0, f);
-  reduce_scatter8(f, x.q, out);
-}
-
-// ---------------------------------------------------------------------------------------
-// Matrix-free apply of the reduced tangent to one periodic vector, streaming the RVE in
-// z-layers: element results of a layer go to shared memory, then every node of the layer
-// gathers its 4 bottom and 4 top contributions in a fixed order.  Returns p . Ap (CTA-wide).
-template <typename T>
-__device__ double apply_tangent(const RvePcgArgs<T>& a, const RveDesc& d, const double* __restrict__ p,
-                                double* __restrict__ Ap, double* smem, double* scratch, const T* gtab) {
-  const int nxy = d.nx * d.ny;
-  double* ye = smem;                  // nxy * 24
-  double* acc_cur = ye + 24 * nxy;    // nxy * 3
-  double* acc_next = acc_cur + 3 * nxy;
-  double* acc_first = acc_next + 3 * nxy;
-  const T jw = (T)(d.hx * d.hy * d.hz / 8.0);
-  double pap[1] = {0.0};
-  const int items = 8 * nxy;
-  const int rounds = (items + blockDim.x - 1) / blockDim.x;
-  for (int k = 0; k < d.nz; ++k) {
-    ApplyItem<T> cur, nxt;
-    fetch_item(a, d, p, items, nxy, k, 0, cur);
-    fetch_tangent(a, cur);
-    for (int it = 0; it < rounds; ++it) {
-      if (it + 1 < rounds) fetch_item(a, d, p, items, nxy, k, it + 1, nxt);
-      T out[3];
-      apply_item(a, cur, gtab, jw, out);
-      if (cur.live)
-#pragma unroll
-        for (int dd = 0; dd < 3; ++dd) ye[(8 * cur.el + cur.q) * 3 + dd] = (double)out[dd];
-      if (it + 1 < rounds) {
-        fetch_tangent(a, nxt);
-        cur = nxt;
-      }
-    }
-    __syncthreads();
-    for (int n = threadIdx.x; n < nxy; n += blockDim.x) {
-      const int j = n / d.nx, i = n - j * d.nx;
-      double bot[3] = {0, 0, 0}, top[3] = {0, 0, 0};
-      for (int s = 0; s < 4; ++s) {
-        const int di = s & 1, dj = s >> 1;
-        const int el = wrap_down(i - di, d.nx) + d.nx * wrap_down(j - dj, d.ny);
-#pragma unroll
-        for (int dd = 0; dd < 3; ++dd) {
-          bot[dd] += ye[(8 * el + s) * 3 + dd];
-          top[dd] += ye[(8 * el + s + 4) * 3 + dd];
-        }
-      }
-      if (k == 0) {
-#pragma unroll
-        for (int dd = 0; dd < 3; ++dd) acc_first[3 * n + dd] = bot[dd];
-      } else {
-        const int64_t node = d.eoff + n + (int64_t)nxy * k;
-#pragma unroll
-        for (int dd = 0; dd < 3; ++dd) {
-          const double v = acc_cur[3 * n + dd] + bot[dd];
-          Ap[3 * node + dd] = v;
-          pap[0] += p[3 * node + dd] * v;
-        }
-      }
-      if (k == d.nz - 1) {
-        const int64_t node = d.eoff + n;
-#pragma unroll
-        for (int dd = 0; dd < 3; ++dd) {
-          const double v = (n == 0) ? 0.0 : acc_first[3 * n + dd] + top[dd];
-          Ap[3 * node + dd] = v;
-          pap[0] += p[3 * node + dd] * v;
-        }
-      } else {
-#pragma unroll
-        for (int dd = 0; dd < 3; ++dd) acc_next[3 * n + dd] = top[dd];
-      }
-    }
-    __syncthreads();
-    double* t = acc_cur;
-    acc_cur = acc_next;
-    acc_next = t;
-  }
-  block_sum<1>(pap, scratch);
-  return pap[0];
-}
-
-// Jacobi-PCG on one reduced periodic system per CTA: K x = b, x0 = 0.  Bounded iterations;
-// status 0 converged (||r|| <= rtol ||b|| or ||b|| == 0), 1 iteration limit, 2 breakdown
-// (p.Ap <= 0 or non-finite).  Two CTAs per SM in both precisions: the FP64 build then fits
-// 128 registers with ~140 B of spills, and the second CTA hides more of the latency of the
-// per-layer barriers and reductions (2,048 8^3 systems: 23 % less time than at 252
-// registers and one CTA per SM, bitwise the same results).
-template <typename T>
-__global__ void __launch_bounds__(RVE_THREADS, 2) rve_pcg_kernel(const RvePcgArgs<T> a) {
-  extern __shared__ double smem[];
-  __shared__ double scratch[64];
-  const int s = blockIdx.x;
-  const int r = a.sys_rve[s];
-  if (a.active && !a.active[r]) return;
-  const RveDesc d = a.desc[r];
-  const int64_t E = (int64_t)d.nx * d.ny * d.nz;
-  const int64_t off = a.sys_off[s];  // vector offset of this system (3 * node base)
-  if (a.vec_len >= 0 && (off < 0 || E < 0 || off + 3 * E > a.vec_len)) {  // uniform over the CTA
-    if (threadIdx.x == 0) {
-      a.status[s] = 3;
-      a.iterations[s] = 0;
-      a.rel_residual[s] = 0.0;
-      a.xnorm[s] = 0.0;
-    }
-    return;
-  }
-  const double* b = a.b + off;
-  double* x = a.x + off;
-  double* rr = a.r + off;
-  double* p = a.p + off;
-  double* Ap = a.Ap + off;
-  const double* dinv = a.dinv + 3 * d.eoff;
-  __shared__ T gtab[24 * 8];
-  fill_grad_table(d, gtab);  // visible after the block sum below
-  // Shift the vector pointers so that batch node indices address them directly.
-  const int64_t shift = 3 * d.eoff;
-  double* x_ = x - shift;
-  double* r_ = rr - shift;
-  double* p_ = p - shift;
-  double* Ap_ = Ap - shift;
-  double v[2] = {0.0, 0.0};  // rz, bb
-  for (int64_t n = threadIdx.x; n < 3 * E; n += blockDim.x) {
-    const double bi = b[n];
-    x[n] = 0.0;
-    rr[n] = bi;
-    const double z = dinv[n] * bi;
-    p[n] = z;
-    v[0] += bi * z;
-    v[1] += bi * bi;
-  }
-  block_sum<2>(v, scratch);
-  double rz = v[0];
-  const double bnorm = sqrt(v[1]);
-  const double tol = (a.rtol_dev ? *a.rtol_dev : a.rtol) * bnorm;
-  int status = 1, iters = 0;
-  double rnorm = bnorm;
-  if (bnorm == 0.0 || !(bnorm == bnorm)) {
-    status = (bnorm == 0.0) ? 0 : 2;
-  } else {
-    for (iters = 0; iters < a.maxit;) {
-      const double pap = apply_tangent<T>(a, d, p_, Ap_, smem, scratch, gtab);
-      if (!(pap > 0.0) || !isfinite(pap)) {
-        status = 2;
-        break;
-      }
-      const double alpha = rz / pap;
-      double w2[2] = {0.0, 0.0};  // r.r, r.z
-      for (int64_t n = threadIdx.x; n < 3 * E; n += blockDim.x) {
-        x[n] += alpha * p[n];
-        const double rn = rr[n] - alpha * Ap[n];
-        rr[n] = rn;
-        w2[0] += rn * rn;
-        w2[1] += rn * dinv[n] * rn;
-      }
-      block_sum<2>(w2, scratch);
-      ++iters;
-      rnorm = sqrt(w2[0]);
-      if (!isfinite(rnorm)) {
-        status = 2;
-        break;
-      }
-      if (rnorm <= tol) {
-        status = 0;
-        break;
-      }
-      const double beta = w2[1] / rz;
-      rz = w2[1];
-      for (int64_t n = threadIdx.x; n < 3 * E; n += blockDim.x) p[n] = dinv[n] * rr[n] + beta * p[n];
-      __syncthreads();
-    }
-  }
-  double xn[1] = {0.0};
-  for (int64_t n = threadIdx.x; n < 3 * E; n += blockDim.x) xn[0] += x[n] * x[n];
-  block_sum<1>(xn, scratch);
-  if (threadIdx.x == 0) {
-    a.status[s] = status;
-    a.iterations[s] = iters;
-    a.rel_residual[s] = bnorm > 0.0 ? rnorm / bnorm : 0.0;
-    a.xnorm[s] = sqrt(xn[0]);
-  }
-  (void)x_;
-  (void)r_;
-}
-
-// ---------------------------------------------------------------------------------------
-// Cluster variant of the PCG: C CTAs of one thread-block cluster share one system.  Rank q
-// owns the node layers [k0, k1) = [q nz / C, (q + 1) nz / C) of its RVE: it streams its
-// element layers like apply_tangent, keeps the bottom contributions of its first node layer
-// (acc_first) and exports the top contributions of its last element layer, which belong to
-// the next rank's first node layer (the last rank's wrap to node layer 0 is the periodic
-// closure); after a cluster barrier every rank adds its predecessor's export through
-// distributed shared memory.  Dot products are CTA sums combined over the ranks in rank
-// order (every rank forms the same totals, so all ranks take the same branches).  Four
-// cluster barriers per iteration: export, p.Ap, r.r / r.z, and p visibility.  The layer's
-// element contributions are kept in the element type T (exact: they are computed in T),
-// the node sums in double as in rve_pcg_kernel; in FP32 mode that is 192 bytes per node of
-// a layer, and with at most 128 registers two CTAs fit on an SM.
-template <typename T>
-__device__ double apply_tangent_slab(const RvePcgArgs<T>& a, const RveDesc& d, const double* __restrict__ p,
-                                     double* __restrict__ Ap, unsigned char* smem, int k0, int k1,
-                                     cg::cluster_group& cl, unsigned prev_rank,
-                                     const T* gtab) {
-  const int nxy = d.nx * d.ny;
-  T* ye = reinterpret_cast<T*>(smem);  // nxy * 24 element-node contributions of one layer (exact in T)
-  double* acc_cur = reinterpret_cast<double*>(smem + (size_t)24 * nxy * sizeof(T));  // nxy * 3 node sums
-  double* acc_next = acc_cur + 3 * nxy;
-  double* acc_first = acc_next + 3 * nxy;
-  double* exported = acc_first + 3 * nxy;
-  const T jw = (T)(d.hx * d.hy * d.hz / 8.0);
-  double pap = 0.0;
-  const int items = 8 * nxy;
-  const int rounds = (items + blockDim.x - 1) / blockDim.x;
-  for (int k = k0; k < k1; ++k) {
-    ApplyItem<T> cur, nxt;
-    fetch_item(a, d, p, items, nxy, k, 0, cur);
-    fetch_tangent(a, cur);
-    for (int it = 0; it < rounds; ++it) {
-      if (it + 1 < rounds) fetch_item(a, d, p, items, nxy, k, it + 1, nxt);
-      T out[3];
-      apply_item(a, cur, gtab, jw, out);
-      if (cur.live)
-#pragma unroll
-        for (int dd = 0; dd < 3; ++dd) ye[(8 * cur.el + cur.q) * 3 + dd] = out[dd];
-      if (it + 1 < rounds) {
-        fetch_tangent(a, nxt);
-        cur = nxt;
-      }
-    }
-    __syncthreads();
-    for (int n = threadIdx.x; n < nxy; n += blockDim.x) {
-      const int j = n / d.nx, i = n - j * d.nx;
-      double bot[3] = {0, 0, 0}, top[3] = {0, 0, 0};
-      for (int s = 0; s < 4; ++s) {
-        const int di = s & 1, dj = s >> 1;
-        const int el = wrap_down(i - di, d.nx) + d.nx * wrap_down(j - dj, d.ny);
-#pragma unroll
-        for (int dd = 0; dd < 3; ++dd) {
-          bot[dd] += (double)ye[(8 * el + s) * 3 + dd];
-          top[dd] += (double)ye[(8 * el + s + 4) * 3 + dd];
-        }
-      }
-      if (k == k0) {
-#pragma unroll
-        for (int dd = 0; dd < 3; ++dd) acc_first[3 * n + dd] = bot[dd];
-      } else {
-        const int64_t node = d.eoff + n + (int64_t)nxy * k;
-#pragma unroll
-        for (int dd = 0; dd < 3; ++dd) {
-          const double v = acc_cur[3 * n + dd] + bot[dd];
-          Ap[3 * node + dd] = v;
-          pap += p[3 * node + dd] * v;
-        }
-      }
-      if (k == k1 - 1) {
-#pragma unroll
-        for (int dd = 0; dd < 3; ++dd) exported[3 * n + dd] = top[dd];
-      } else {
-#pragma unroll
-        for (int dd = 0; dd < 3; ++dd) acc_next[3 * n + dd] = top[dd];
-      }
-    }
-    __syncthreads();
-    double* t = acc_cur;
-    acc_cur = acc_next;
-    acc_next = t;
-  }
-  cl.sync();  // every rank's export is complete
-  const double* prev = cl.map_shared_rank(exported, prev_rank);
-  for (int n = threadIdx.x; n < nxy; n += blockDim.x) {
-    const int64_t node = d.eoff + n + (int64_t)nxy * k0;
-#pragma unroll
-    for (int dd = 0; dd < 3; ++dd) {
-      const double v = (k0 == 0 && n == 0) ? 0.0 : acc_first[3 * n + dd] + prev[3 * n + dd];
-      Ap[3 * node + dd] = v;
-      pap += p[3 * node + dd] * v;
-    }
-  }
-  return pap;
-}
-
-// Sum of NV doubles over the CTAs of the cluster, the same on every thread of every rank.
-// `slots` (NV doubles of this CTA's shared memory) must not be rewritten before the next
-// cluster barrier that follows every rank's read.
-template <int NV>
-__device__ __forceinline__ void cluster_sum(double (&v)[NV], double* scratch, double* slots, cg::cluster_group& cl) {
-  block_sum<NV>(v, scratch);
-  if (threadIdx.x == 0)
-#pragma unroll
-    for (int k = 0; k < NV; ++k) slots[k] = v[k];
-  cl.sync();
-  double t[NV];
-#pragma unroll
-  for (int k = 0; k < NV; ++k) t[k] = 0.0;
-  const unsigned nr = cl.num_blocks();
-  for (unsigned q = 0; q < nr; ++q) {
-    const double* rem = cl.map_shared_rank(slots, q);
-#pragma unroll
-    for (int k = 0; k < NV; ++k) t[k] += rem[k];
-  }
-#pragma unroll
-  for (int k = 0; k < NV; ++k) v[k] = t[k];
-}
-
-// Launch shapes of the cluster PCG (threads per CTA, resident CTAs per SM -> register cap),
-// chosen per batch by the tuner: 0 is the default, 1-3 trade threads for registers.
-template <typename T, int SHAPE>
-struct PcgShape;
-template <typename T>
-struct PcgShape<T, 0> {
-  static constexpr int threads = 256, min_blocks = sizeof(T) == 4 ? 2 : 1;
-};
-template <typename T>
-struct PcgShape<T, 1> {
-  static constexpr int threads = 128, min_blocks = sizeof(T) == 4 ? 4 : 2;
-};
-template <typename T>
-struct PcgShape<T, 2> {
-  static constexpr int threads = 512, min_blocks = 1;
-};
-template <typename T>
-struct PcgShape<T, 3> {
-  static constexpr int threads = 256, min_blocks = sizeof(T) == 4 ? 1 : 2;
-};
-
-template <typename T, int SHAPE>
-__global__ void __launch_bounds__(PcgShape<T, SHAPE>::threads, PcgShape<T, SHAPE>::min_blocks)
-    rve_pcg_cluster_kernel(const RvePcgArgs<T> a) {
-  extern __shared__ double smem_dyn[];  // the layer buffers of apply_tangent_slab
-  unsigned char* smem = reinterpret_cast<unsigned char*>(smem_dyn);
-  __shared__ double scratch[64];
-  __shared__ double slot_init[2], slot_pap[1], slot_rr[2], slot_xn[1];
-  cg::cluster_group cl = cg::this_cluster();
-  const unsigned C = cl.num_blocks();
-  const unsigned rank = cl.block_rank();
-  const int s = blockIdx.x / C;
-  const int r = a.sys_rve[s];
-  if (a.active && !a.active[r]) return;  // the whole cluster leaves together
-  const RveDesc d = a.desc[r];
-  if (d.nz < (int)C) {  // every rank must own a layer
-    if (rank == 0 && threadIdx.x == 0) {
-      a.status[s] = 3;
-      a.iterations[s] = 0;
-      a.rel_residual[s] = 0.0;
-      a.xnorm[s] = 0.0;
-    }
-    return;
-  }
-  const int nxy = d.nx * d.ny;
-  __shared__ T gtab[24 * 8];
-  fill_grad_table(d, gtab);  // visible after the first cluster sum
-  const int k0 = (int)((rank * (unsigned)d.nz) / C), k1 = (int)(((rank + 1) * (unsigned)d.nz) / C);
-  const unsigned prev_rank = (rank + C - 1) % C;
-  const int64_t off = a.sys_off[s];
-  const int64_t shift = 3 * d.eoff;
-  const int64_t lo = 3 * (int64_t)nxy * k0, hi = 3 * (int64_t)nxy * k1;  // this rank's vector entries
-  const double* b = a.b + off;
-  double* x = a.x + off;
-  double* rr = a.r + off;
-  double* p = a.p + off;
-  double* Ap = a.Ap + off;
-  const double* dinv = a.dinv + 3 * d.eoff;
-  double v[2] = {0.0, 0.0};  // r.z, b.b
-  for (int64_t n = lo + threadIdx.x; n < hi; n += blockDim.x) {
-    const double bi = b[n];
-    x[n] = 0.0;
-    rr[n] = bi;
-    const double z = dinv[n] * bi;
-    p[n] = z;
-    v[0] += bi * z;
-    v[1] += bi * bi;
-  }
-  cluster_sum<2>(v, scratch, slot_init, cl);  // its barrier also publishes p
-  double rz = v[0];
-  const double bnorm = sqrt(v[1]);
-  const double tol = (a.rtol_dev ? *a.rtol_dev : a.rtol) * bnorm;
-  int status = 1, iters = 0;
-  double rnorm = bnorm;
-  if (bnorm == 0.0 || !(bnorm == bnorm)) {
-    status = (bnorm == 0.0) ? 0 : 2;
-  } else {
-    for (iters = 0; iters < a.maxit;) {
-      double pap[1] = {apply_tangent_slab<T>(a, d, p - shift, Ap - shift, smem, k0, k1, cl, prev_rank, gtab)};
-      cluster_sum<1>(pap, scratch, slot_pap, cl);
-      if (!(pap[0] > 0.0) || !isfinite(pap[0])) {
-        status = 2;
-        break;
-      }
-      const double alpha = rz / pap[0];
-      double w2[2] = {0.0, 0.0};  // r.r, r.z
-      for (int64_t n = lo + threadIdx.x; n < hi; n += blockDim.x) {
-        x[n] += alpha * p[n];
-        const double rn = rr[n] - alpha * Ap[n];
-        rr[n] = rn;
-        w2[0] += rn * rn;
-        w2[1] += rn * dinv[n] * rn;
-      }
-      cluster_sum<2>(w2, scratch, slot_rr, cl);
-      ++iters;
-      rnorm = sqrt(w2[0]);
-      if (!isfinite(rnorm)) {
-        status = 2;
-        break;
-      }
-      if (rnorm <= tol) {
-        status = 0;
-        break;
-      }
-      const double beta = w2[1] / rz;
-      rz = w2[1];
-      for (int64_t n = lo + threadIdx.x; n < hi; n += blockDim.x) p[n] = dinv[n] * rr[n] + beta * p[n];
-      cl.sync();  // p of every rank visible before the next apply
-    }
-  }
-  double xn[1] = {0.0};
-  for (int64_t n = lo + threadIdx.x; n < hi; n += blockDim.x) xn[0] += x[n] * x[n];
-  cluster_sum<1>(xn, scratch, slot_xn, cl);
-  if (rank == 0 && threadIdx.x == 0) {
-    a.status[s] = status;
-    a.iterations[s] = iters;
-    a.rel_residual[s] = bnorm > 0.0 ? rnorm / bnorm : 0.0;
-    a.xnorm[s] = sqrt(xn[0]);
-  }
-  cl.sync();  // no rank leaves while another may still read its shared memory
-}
-
-// ---------------------------------------------------------------------------------------
 // Right-hand sides of the effective-tangent solves and K_ee.  For macro strain unit j,
 // element forces f_e^(j) = sum_q w B_q^T C_q e_j; gathered periodically they give column j
 // of K_we = T^T K A; K_ee = A^T K A = sum_q w C_q (since B_q A e_j = e_j on a box).
@@ -1435,55 +902,6 @@ int launch_rve_gather(const RveGatherArgs& a, int nrve, cudaStream_t st) {
 }
 
 template <typename T>
-int launch_rve_pcg(const RvePcgArgs<T>& a, int nsys, int max_nxy, cudaStream_t st) {
-  const size_t smem = (size_t)max_nxy * (24 + 9) * sizeof(double);
-  if (smem > 200 * 1024) return CIB_ERANGE;
-  const int rc = allow_dynamic_smem(reinterpret_cast<const void*>(rve_pcg_kernel<T>), 200 * 1024);
-  if (rc != CIB_OK) return rc;
-  rve_pcg_kernel<T><<<nsys, RVE_THREADS, smem, st>>>(a);
-  return check_launch();
-}
-
-template <typename T, int SHAPE>
-int launch_rve_pcg_cluster_shape(const RvePcgArgs<T>& a, int nsys, int cluster, size_t smem, cudaStream_t st) {
-  const void* fn = reinterpret_cast<const void*>(rve_pcg_cluster_kernel<T, SHAPE>);
-  const int rc = allow_dynamic_smem(fn, 200 * 1024);
-  if (rc != CIB_OK) return rc;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)nsys * (unsigned)cluster, 1, 1);
-  cfg.blockDim = dim3(PcgShape<T, SHAPE>::threads, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)cluster;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, rve_pcg_cluster_kernel<T, SHAPE>, a);
-  return check_launch();
-}
-
-// cluster: the CTAs per system (1, 2, 4 or 8) in bits 0-3 and the launch shape (0-3, see
-// PcgShape) in bits 4-7; cluster size 1 is the one-CTA kernel, whatever the shape.
-template <typename T>
-int launch_rve_pcg_cluster(const RvePcgArgs<T>& a, int nsys, int max_nxy, int cluster, cudaStream_t st) {
-  const int c = cluster & 15, shape = (cluster >> 4) & 15;
-  if ((cluster >> 8) != 0 || shape > 3) return CIB_EINVAL;
-  if (c == 1) return launch_rve_pcg<T>(a, nsys, max_nxy, st);
-  if (c != 2 && c != 4 && c != 8) return CIB_EINVAL;
-  const size_t smem = (size_t)max_nxy * (24 * sizeof(T) + 12 * sizeof(double));
-  if (smem > 200 * 1024) return CIB_ERANGE;
-  switch (shape) {
-    case 1: return launch_rve_pcg_cluster_shape<T, 1>(a, nsys, c, smem, st);
-    case 2: return launch_rve_pcg_cluster_shape<T, 2>(a, nsys, c, smem, st);
-    case 3: return launch_rve_pcg_cluster_shape<T, 3>(a, nsys, c, smem, st);
-    default: return launch_rve_pcg_cluster_shape<T, 0>(a, nsys, c, smem, st);
-  }
-}
-
-template <typename T>
 int launch_rve_tangent_rhs(const RveTangentArgs<T>& a, int nrve, cudaStream_t st) {
   rve_tangent_rhs_kernel<T><<<nrve, RVE_THREADS, 0, st>>>(a);
   return check_launch();
@@ -1502,10 +920,6 @@ int launch_rve_response(const RveResponseArgs<T>& a, int nrve, cudaStream_t st) 
 
 template int launch_rve_residual<float>(const RveResidualArgs<float>&, int, cudaStream_t);
 template int launch_rve_residual<double>(const RveResidualArgs<double>&, int, cudaStream_t);
-template int launch_rve_pcg<float>(const RvePcgArgs<float>&, int, int, cudaStream_t);
-template int launch_rve_pcg<double>(const RvePcgArgs<double>&, int, int, cudaStream_t);
-template int launch_rve_pcg_cluster<float>(const RvePcgArgs<float>&, int, int, int, cudaStream_t);
-template int launch_rve_pcg_cluster<double>(const RvePcgArgs<double>&, int, int, int, cudaStream_t);
 template int launch_rve_tangent_rhs<float>(const RveTangentArgs<float>&, int, cudaStream_t);
 template int launch_rve_tangent_rhs<double>(const RveTangentArgs<double>&, int, cudaStream_t);
 template int launch_rve_response<float>(const RveResponseArgs<float>&, int, cudaStream_t);

@@ -502,7 +502,7 @@ class RVEBatch:
 
     def pcg_launch(self) -> int:
         """The ``cluster`` argument of cib_rve_pcg_cluster: CTAs per system in bits 0-3, the
-        launch shape (threads per CTA / register cap) in bits 4-7."""
+        launch shape (threads per CTA) in bits 4-7."""
         return int(self.cluster) | (int(self.pcg_shape) << 4)
 
     def check_cluster(self, cluster: int) -> int:
@@ -856,8 +856,8 @@ def auto_pcg_cluster(batch: RVEBatch) -> int:
     return c
 
 
-PCG_SHAPES = {0: "256 threads, default register cap", 1: "128 threads, 4 (FP64: 2) CTAs per SM",
-              2: "512 threads, 1 CTA per SM", 3: "256 threads, the other register cap (FP32: 1, FP64: 2 CTAs per SM)"}
+PCG_SHAPES = {0: "256 threads (FP64: 128 or 256 by the grid)", 1: "128 threads", 2: "512 threads (FP64: 256)",
+              3: "256 threads (FP64: 64)"}
 
 
 def _tuning_path() -> Path:
@@ -881,7 +881,7 @@ def tune_pcg_cluster(batch: RVEBatch, update_settings: MaterialUpdateSettings, c
                      shapes=(0, 1, 2, 3), persist: bool = True) -> dict:  # fmt: skip
     """Time one PCG solve of the batch's current Newton system (a residual pass at the
     committed fluctuation) for every admissible cluster size x launch shape (threads per
-    CTA and register cap, ``PCG_SHAPES``; shapes apply to cluster sizes above 1) and keep
+    CTA, ``PCG_SHAPES``; shapes apply to cluster sizes above 1) and keep
     the fastest.  The solves write only work vectors; the batch's state is unchanged.
     With ``persist`` the choice is stored per edge mix (precision, GPU, RVE divisions) in
     a JSON file (``$CIB_TUNING_CACHE``, else ``~/.cache/cib200/pcg_tuning.json``) and a

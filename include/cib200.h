@@ -314,13 +314,13 @@ int cib_rve_pcg(const cib_rve_batch* batch, int32_t nsys, const int32_t* sys_rve
 
 /* cib_rve_pcg with `cluster` (1, 2, 4 or 8) CTAs of one thread-block cluster per system:
  * each CTA owns a slab of z node layers, slab boundaries are exchanged and the dot
- * products combined through distributed shared memory (fixed rank order, so results are
- * reproducible for a given cluster size).  Every RVE needs nz >= cluster (else that
- * system's status is 3); cluster 1 is cib_rve_pcg.  Bits 4-7 of `cluster` select the launch
- * shape of the cluster kernel (threads per CTA / CTAs per SM, which caps the registers):
- * 0 the default (256 / 2 in FP32, 256 / 1 in FP64), 1 (128 / 4 FP32, 128 / 2 FP64),
- * 2 (512 / 1), 3 (256 / 1 FP32, 256 / 2 FP64); results do not depend on the shape beyond
- * rounding of the CTA sums.  Same reference interface as cib_rve_pcg (Tᵀ K T + spsolve,
+ * products combined through distributed shared memory in a fixed order.  Every RVE needs
+ * nz >= cluster (else that system's status is 3); cluster 1 is cib_rve_pcg.  Bits 4-7 of
+ * `cluster` select the threads per CTA: 0 the default (256 in FP32; 128 or 256 by the grid in
+ * FP64), 1 128, 2 512 in FP32 and 256 in FP64, 3 256 in FP32 and 64 in FP64.  FP64 results are
+ * bitwise the same for every cluster size and shape (a grid that would leave SMs idle gets up
+ * to 8 CTAs per system whatever `cluster` asks for); FP32 results are reproducible for given
+ * ones.  Same reference interface as cib_rve_pcg (Tᵀ K T + spsolve,
  * src/fem/rve/solver.py:143-144). */
 int cib_rve_pcg_cluster(const cib_rve_batch* batch, int32_t nsys, const int32_t* sys_rve, const int64_t* sys_off,
                         const int32_t* active, const double* b, const double* dinv, double* x, double* r, double* p,
