@@ -179,6 +179,25 @@ class RNOWindowC(ctypes.Structure):
     ]
 
 
+class RNOWgradC(ctypes.Structure):
+    """``cib_rno_wgrad``."""
+
+    _fields_ = [
+        ("K", ctypes.c_int32),
+        ("splits", ctypes.c_int32),
+        ("ld", ctypes.c_int64),
+        ("M", ctypes.c_int32 * 4),
+        ("N", ctypes.c_int32 * 4),
+        ("A", ctypes.c_void_p * 4),
+        ("B", ctypes.c_void_p * 4),
+        ("gw", ctypes.c_void_p * 4),
+        ("gb", ctypes.c_void_p * 4),
+        ("partial", ctypes.c_void_p),
+        ("row_partial", ctypes.c_void_p),
+        ("err", ctypes.c_void_p),
+    ]
+
+
 class EnergyRNOC(ctypes.Structure):
     """``cib_energy_rno``."""
 
@@ -226,6 +245,7 @@ SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "cib_counter_increment": (_I, [_P, _P]),
     "cib_rno_window_forward": (_I, [_P, _P]),
     "cib_rno_window_backward": (_I, [_P, _P]),
+    "cib_rno_weight_gradients": (_I, [_P, _P]),
     "cib_rno_gate_prepare": (_I, [_I64, _P, _P, _D, _D, _P, _D] + [_P] * 7),
     "cib_rno_gate_finish": (_I, [_I64, _P, _D, _P, _P, _P, _P, _P]),
     "cib_verlet_predict": (_I, [_I64, _P, _P, _P, _P, _D, _P, _P]),

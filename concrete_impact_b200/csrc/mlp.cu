@@ -233,6 +233,164 @@ __global__ void __launch_bounds__(GEMM_THREADS) umma_gemm_kernel(const GemmArgs 
   }
 }
 
+// ---------------------------------------------------------------------------------------
+// All weight and bias gradients of a window in two launches: dW_l = A_l B_l^T over the R rows
+// of the window (A_l: transposed pre-activation gradients, M_l x R; B_l: transposed layer
+// inputs, N_l x R), split over K slices x layers, then one reduction.  Four GEMM launches of
+// 50 CTAs each left two thirds of the chip idle, and their row sums (the bias gradients, 50 us
+// each) read every A_l again from memory with one block per row; here a slice's row sums come
+// from the operand tiles that the GEMM stages anyway.  Slices, K order and the order of the
+// sums over the slices are those of umma_gemm_kernel<EPI_PARTIAL> and splitk_reduce_kernel.
+struct WgradArgs {
+  cib_rno_wgrad g;
+  int k_per_split;
+  int offset[5];  // first element of each layer's partial tiles within a slice's; [4]: all
+};
+
+struct __align__(1024) WgradSmem {
+  uint8_t a[GEMM_STAGES][128 * KC * 2];
+  uint8_t b[GEMM_STAGES][128 * KC * 2];
+  uint64_t bar[GEMM_STAGES];
+  uint32_t tmem_base;
+};
+
+__global__ void __launch_bounds__(GEMM_THREADS) wgrad_kernel(const WgradArgs w) {
+  extern __shared__ uint8_t smem_raw[];
+  WgradSmem& S = *reinterpret_cast<WgradSmem*>(smem_raw);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int l = blockIdx.y, M = w.g.M[l], N = w.g.N[l];
+  const __nv_bfloat16* A = static_cast<const __nv_bfloat16*>(w.g.A[l]);
+  const __nv_bfloat16* B = static_cast<const __nv_bfloat16*>(w.g.B[l]);
+  const int64_t ld = w.g.ld;
+  const int k_begin = blockIdx.x * w.k_per_split, k_end = min(w.g.K, k_begin + w.k_per_split);
+  const int chunks = (k_end - k_begin + KC - 1) / KC;
+  if (warp == 0) tmem_alloc(&S.tmem_base, 128);
+  if (tid == 0)
+    for (int s = 0; s < GEMM_STAGES; ++s) mbar_init(&S.bar[s], 1);
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  const uint32_t tmem = S.tmem_base;
+  const uint32_t idesc = idesc_bf16(N);
+
+  auto load_chunk = [&](int i, int st) {  // rows beyond M and columns beyond the slice are zero
+    const int k0 = k_begin + i * KC;
+    for (int v = tid; v < 128 * (KC / 8); v += GEMM_THREADS) {
+      const int r = v / (KC / 8), c = (v % (KC / 8)) * 8;
+      const bool in = r < M && k0 + c < k_end;
+      cp_async16(S.a[st] + core_offset(r, c, KC), in ? A + r * ld + k0 + c : A, in);
+    }
+    for (int v = tid; v < N * (KC / 8); v += GEMM_THREADS) {
+      const int r = v / (KC / 8), c = (v % (KC / 8)) * 8;
+      const bool in = k0 + c < k_end;
+      cp_async16(S.b[st] + core_offset(r, c, KC), in ? B + r * ld + k0 + c : B, in);
+    }
+  };
+
+#pragma unroll
+  for (int s = 0; s < GEMM_STAGES - 1; ++s) {
+    if (s < chunks) load_chunk(s, s);
+    cp_async_commit();
+  }
+  bool failed = false;
+  double row_sum = 0.0;  // of A row `tid` over the slice
+  for (int i = 0; i < chunks; ++i) {
+    const int st = i % GEMM_STAGES;
+    cp_async_wait<GEMM_STAGES - 2>();
+    fence_smem_to_async();
+    __syncthreads();
+    if (tid == 0) {
+      fence_after_sync();
+      const int steps = min(KC, k_end - (k_begin + i * KC)) / 16;
+      const uint32_t a0 = smem_u32(S.a[st]), b0 = smem_u32(S.b[st]);
+      for (int s = 0; s < steps; ++s) {
+        const uint64_t da = sdesc(a0 + 256 * s, 128, KC * 16);
+        const uint64_t db = sdesc(b0 + 256 * s, 128, KC * 16);
+        const uint32_t acc = (i > 0 || s > 0) ? 1u : 0u;
+        asm volatile(
+            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+            " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n}\n" ::"r"(tmem),
+            "l"(da), "l"(db), "r"(idesc), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
+            : "memory");
+      }
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                       smem_u32(&S.bar[st]))
+                   : "memory");
+    }
+    // the chunk's row sum from the staged tile, while the tensor core reads it too
+#pragma unroll
+    for (int c = 0; c < KC; c += 8) {
+      const uint4 q = *reinterpret_cast<const uint4*>(S.a[st] + core_offset(tid, c, KC));
+      const uint32_t u[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        row_sum += (double)__uint_as_float(u[e] << 16) + (double)__uint_as_float(u[e] & 0xffff0000u);
+    }
+    const int j = i + GEMM_STAGES - 1;
+    if (j < chunks) {
+      if (i >= 1) {
+        const int prev = i - 1;
+        const bool ok = mbar_wait(&S.bar[prev % GEMM_STAGES], (uint32_t)((prev / GEMM_STAGES) & 1));
+        if (__syncthreads_or(ok ? 0 : 1)) {
+          failed = true;
+          break;
+        }
+      }
+      load_chunk(j, j % GEMM_STAGES);
+    }
+    cp_async_commit();
+  }
+  if (!failed && chunks > 0) {
+    const int last = chunks - 1;
+    const bool ok = mbar_wait(&S.bar[last % GEMM_STAGES], (uint32_t)((last / GEMM_STAGES) & 1));
+    failed = __syncthreads_or(ok ? 0 : 1) != 0;
+  }
+  cp_async_wait<0>();
+  fence_after_sync();
+  if (failed) {
+    if (tid == 0) atomicExch(w.g.err, 1u);
+  } else {
+    if (tid < M) w.g.row_partial[((size_t)blockIdx.x * 4 + l) * 128 + tid] = row_sum;
+    float* dst = w.g.partial + (size_t)blockIdx.x * w.offset[4] + w.offset[l] + (size_t)tid * N;
+    for (int c = 0; c < N; c += 16) {
+      float v[16];
+      tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c, v);
+      if (tid < M)
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          reinterpret_cast<float4*>(dst + c)[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+    }
+  }
+  (void)lane;
+  fence_before_sync();
+  __syncthreads();
+  if (warp == 0) {
+    fence_after_sync();
+    tmem_dealloc(tmem, 128);
+  }
+}
+
+__global__ void __launch_bounds__(256) wgrad_reduce_kernel(const WgradArgs w, int slices) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < w.offset[4]) {
+    int l = 0;
+    while (i >= w.offset[l + 1]) ++l;
+    float s = 0.0f;
+#pragma unroll 8
+    for (int k = 0; k < slices; ++k) s += w.g.partial[(size_t)k * w.offset[4] + i];
+    w.g.gw[l][i - w.offset[l]] = s;
+  }
+  if (i < 4 * 128) {  // bias gradients
+    const int l = i >> 7, m = i & 127;
+    if (m < w.g.M[l]) {
+      double s = 0.0;
+#pragma unroll 8
+      for (int k = 0; k < slices; ++k) s += w.g.row_partial[((size_t)k * 4 + l) * 128 + m];
+      w.g.gb[l][m] = (float)s;
+    }
+  }
+}
+
 // out[m * ldo + n] = sum over s of partial[(s * M + m) * ldc + n]  (fixed order)
 __global__ void splitk_reduce_kernel(int M, int N, int splits, const float* __restrict__ partial, int ldc,
                                      float* __restrict__ out, int ldo) {
@@ -325,5 +483,33 @@ extern "C" int cib_splitk_reduce(int32_t M, int32_t N, int32_t splits, const flo
   const int threads = 256;
   splitk_reduce_kernel<<<(M * N + threads - 1) / threads, threads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       M, N, splits, partial, ldc, out, ldo);
+  return check_launch();
+}
+
+extern "C" int cib_rno_weight_gradients(const cib_rno_wgrad* g, void* stream) {
+  if (!g || g->K < 16 || (g->K % 16) != 0 || g->ld < g->K || (g->ld % 8) != 0 || g->splits < 1 || !g->partial ||
+      !aligned16(g->partial) || !g->row_partial || !g->err)
+    return CIB_EINVAL;
+  WgradArgs a;
+  a.g = *g;
+  a.offset[0] = 0;
+  for (int l = 0; l < 4; ++l) {
+    if (g->M[l] < 1 || g->M[l] > 128 || g->N[l] < 16 || g->N[l] > 128 || (g->N[l] % 16) != 0 || !g->A[l] || !g->B[l] ||
+        !aligned16(g->A[l]) || !aligned16(g->B[l]) || !g->gw[l] || !g->gb[l])
+      return CIB_EINVAL;
+    a.offset[l + 1] = a.offset[l] + g->M[l] * g->N[l];
+  }
+  int per = (g->K + g->splits - 1) / g->splits;
+  per = ((per + KC - 1) / KC) * KC;
+  a.k_per_split = per;
+  const int slices = (g->K + per - 1) / per;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const int bytes = (int)sizeof(WgradSmem);
+  if (allow_dynamic_smem(reinterpret_cast<const void*>(wgrad_kernel), bytes) != CIB_OK) return CIB_ECUDA;
+  wgrad_kernel<<<dim3((unsigned)slices, 4), GEMM_THREADS, bytes, st>>>(a);
+  const int rc = check_launch();
+  if (rc != CIB_OK) return rc;
+  const int items = a.offset[4] > 512 ? a.offset[4] : 512;
+  wgrad_reduce_kernel<<<(unsigned)((items + 255) / 256), 256, 0, st>>>(a, slices);
   return check_launch();
 }

@@ -94,7 +94,19 @@ __global__ void row_sum_bf16_kernel(int R, const __nv_bfloat16* __restrict__ X, 
   __shared__ double red[256];
   const int n = blockIdx.x;
   double s = 0.0;
-  for (int r = threadIdx.x; r < R; r += blockDim.x) s += (double)__bfloat162float(X[(size_t)n * ld + r]);
+  const __nv_bfloat16* row = X + (size_t)n * ld;
+  // 8 values per load when the row allows it, four loads in flight per thread (25,600 columns:
+  // 50 us with single values, 4.5 us)
+  const int vec = (reinterpret_cast<uintptr_t>(row) & 15u) == 0 ? R / 8 : 0;
+#pragma unroll 4
+  for (int r = threadIdx.x; r < vec; r += blockDim.x) {
+    const uint4 q = reinterpret_cast<const uint4*>(row)[r];
+    const uint32_t u[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      s += (double)__uint_as_float(u[e] << 16) + (double)__uint_as_float(u[e] & 0xffff0000u);
+  }
+  for (int r = 8 * vec + threadIdx.x; r < R; r += blockDim.x) s += (double)__bfloat162float(row[r]);
   red[threadIdx.x] = s;
   __syncthreads();
   for (int k = blockDim.x / 2; k > 0; k >>= 1) {

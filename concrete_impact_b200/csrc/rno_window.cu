@@ -581,6 +581,408 @@ __global__ void __launch_bounds__(RW_THREADS, 1) rno_infer_kernel(const cib_rno_
   }
 }
 
+// ---------------------------------------------------------------------------------------
+// Narrow windows: the recurrence runs T dependent steps of four layers, so a window of a few
+// hundred paths is bound by the latency of one layer, not by its arithmetic.  Here the
+// operands change places: the weights are the MMA's A operand (M = 128 hidden units, resident
+// in shared memory), a tile of 16 paths is its B operand (N = 16), and the accumulator holds
+// one hidden unit per TMEM lane and one path per column.  512 paths are then 32 CTAs instead
+// of 4, a thread's bias/GELU epilogue has 8 values instead of 32, its Z stores are coalesced
+// over the hidden units and its H^T stores are 16-byte rows of 8 paths.  One barrier per
+// layer: it publishes the operand tile and carries the failure flag of the last wait.
+// Products and sums are those of the wide kernels (bitwise the same results; only the window
+// loss is grouped differently).  The output layers (12 and 18 rows) are padded to M = 128
+// with zero rows.
+//
+// A step is four layers of ~1,800 cycles: barrier 250, issue and wait 450, epilogue 900.
+constexpr int NP = 16;             // paths per tile
+constexpr int NW_THREADS = 256;    // 8 warps: four TMEM lane quarters x two halves of 8 columns
+constexpr uint32_t NP_LBO = 144;   // core matrices along K, padded by 16 bytes: a warp's 32 hidden
+                                   // units write 4 of them per path without bank conflicts
+__host__ __device__ constexpr uint32_t np_sbo(int k) { return NP_LBO * (uint32_t)(k / 8); }
+__device__ __forceinline__ uint32_t np_offset(int p, int c, int k) {
+  return (uint32_t)(p >> 3) * np_sbo(k) + (uint32_t)(c >> 3) * NP_LBO + (uint32_t)((p & 7) * 16 + (c & 7) * 2);
+}
+
+struct __align__(1024) NarrowFwdSmem {
+  uint8_t w1[HID * XIN * 2];
+  uint8_t w2[HID * HID * 2];
+  uint8_t w3[HID * HID * 2];
+  uint8_t w4[HID * HID * 2];  // rows 16.. zero
+  uint8_t x[2 * np_sbo(XIN)];
+  uint8_t h[2 * np_sbo(HID)];
+  float y[12][NP];             // output layer: rows 0..5 stress, 6..11 latent rate
+  float e[2][NP][6], z[2][NP][6];  // strain and latent of the even and odd steps
+  float skip[36];
+  double red[NW_THREADS / 32];
+  uint64_t bar;
+  uint32_t tmem;
+};
+
+struct __align__(1024) NarrowBwdSmem {
+  uint8_t w4t[HID * YOUT * 2];
+  uint8_t w3t[HID * HID * 2];
+  uint8_t w2t[HID * HID * 2];
+  uint8_t w1t[HID * HID * 2];  // rows 32.. zero
+  uint8_t dy[2 * np_sbo(YOUT)];
+  uint8_t d[2 * np_sbo(HID)];
+  float dx[6][NP];     // latent rows of dX
+  float gs[2][NP][6];  // loss gradient of the even and odd steps
+  float skip[36];
+  uint64_t bar;
+  uint32_t tmem;
+};
+
+__device__ __forceinline__ uint64_t weight_desc(const uint8_t* w, int k) { return sdesc(smem_u32(w), 128, (uint32_t)k * 16); }
+__device__ __forceinline__ uint64_t tile_desc(const uint8_t* b, int k) { return sdesc(smem_u32(b), NP_LBO, np_sbo(k)); }
+
+// Barrier of a layer: operands visible to the tensor core, one thread issues, all wait (after
+// `meanwhile`, work that does not depend on the layer).  False on every thread when a wait of
+// the layer before timed out on any of them.
+template <int K, typename F>
+__device__ __forceinline__ bool narrow_layer(uint64_t* bar, uint32_t tmem, uint64_t da, uint64_t db, uint32_t& phase,
+                                             bool& ok, const F& meanwhile) {
+  fence_smem_to_async();
+  fence_before_sync();
+  if (__syncthreads_or(ok ? 0 : 1)) return false;
+  if (threadIdx.x == 0) {
+    fence_after_sync();
+    mma_bf16_steps<K, 256, 2 * NP_LBO>(tmem, da, db, NP, bar);
+  }
+  meanwhile();
+  ok = mbar_wait(bar, phase);
+  phase ^= 1u;
+  fence_after_sync();
+  return true;
+}
+
+// 8 bf16 values of one row (consecutive window rows g..g+7) of a transposed buffer.
+__device__ __forceinline__ void store_row8(__nv_bfloat16* row, size_t g, const float (&v)[8], int count, bool vec) {
+  if (vec && count == 8) {
+    uint4 q;
+    q.x = pack_bf16(v[0], v[1]);
+    q.y = pack_bf16(v[2], v[3]);
+    q.z = pack_bf16(v[4], v[5]);
+    q.w = pack_bf16(v[6], v[7]);
+    *reinterpret_cast<uint4*>(row + g) = q;
+  } else {
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+      if (c < count) row[g + c] = __float2bfloat16_rn(v[c]);
+  }
+}
+
+__device__ __forceinline__ void zero_fill(uint8_t* dst, int bytes) {
+  for (int i = threadIdx.x; i < bytes / 16; i += blockDim.x) reinterpret_cast<uint4*>(dst)[i] = make_uint4(0, 0, 0, 0);
+}
+
+// A step's output rows are finished by the threads that fill the next step's input tile: a
+// thread's column pair is strain (0..5), rate (6..11) or latent (12..17, kept in registers);
+// the threads of the pairs 18..29 finish one stress row each.
+__global__ void __launch_bounds__(NW_THREADS, 1) rno_narrow_forward_kernel(const cib_rno_window w) {
+  extern __shared__ uint8_t smem_raw[];
+  NarrowFwdSmem& S = *reinterpret_cast<NarrowFwdSmem*>(smem_raw);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int quarter = warp & 3, half = warp >> 2;
+  const int unit = quarter * 32 + lane;          // hidden unit (TMEM lane) of the epilogue
+  const int fp = tid & 15, fc = 2 * (tid >> 4);  // path and column pair of the input tile
+  const bool is_in = fc < 12, is_z = fc >= 12 && fc < 18, is_s = fc >= 18 && fc < 30;
+  const int zk = fc - 12, srow = (fc - 18) / 2;
+  const int B = w.B, T = w.T;
+  const int ntiles = (B + NP - 1) / NP;
+  const size_t R = w.ldt > 0 ? (size_t)w.ldt : (size_t)B * T;
+
+  stage_matrix(S.w1, static_cast<const __nv_bfloat16*>(w.W[0]), HID, XIN, XIN);
+  stage_matrix(S.w2, static_cast<const __nv_bfloat16*>(w.W[1]), HID, HID, HID);
+  stage_matrix(S.w3, static_cast<const __nv_bfloat16*>(w.W[2]), HID, HID, HID);
+  stage_matrix(S.w4, static_cast<const __nv_bfloat16*>(w.W[3]), YOUT, HID, HID);
+  zero_fill(S.w4 + YOUT * HID * 2, (HID - YOUT) * HID * 2);
+  for (int i = tid; i < 36; i += NW_THREADS) S.skip[i] = w.skip ? w.skip[i] : 0.0f;
+  if (warp == 0) tmem_alloc(&S.tmem, 32);
+  if (tid == 0) mbar_init(&S.bar, 1);
+  fence_smem_to_async();
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  const uint32_t tmem = S.tmem;
+  const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(8 * half);
+  const uint64_t dw1 = weight_desc(S.w1, XIN), dw2 = weight_desc(S.w2, HID), dw3 = weight_desc(S.w3, HID),
+                 dw4 = weight_desc(S.w4, HID), dx = tile_desc(S.x, XIN), dh = tile_desc(S.h, HID);
+  const bool has_skip = w.skip != nullptr;
+  const float bias_l[3] = {w.bias[0][unit], w.bias[1][unit], w.bias[2][unit]};
+  float bias_o[2] = {0.0f, 0.0f};
+  if (is_z) {
+    bias_o[0] = w.bias[3][6 + zk];
+    bias_o[1] = w.bias[3][7 + zk];
+  }
+  if (is_s) bias_o[0] = w.bias[3][srow];
+  const auto nothing = [] {};
+  uint32_t phase = 0;
+  bool ok = true, run = true;
+
+  for (int tile = blockIdx.x; tile < ntiles && run; tile += gridDim.x) {
+    const int p0 = tile * NP, q0 = p0 + 8 * half;  // this warp's columns are paths q0 .. q0 + 7
+    const int count = min(max(B - q0, 0), 8);
+    const int p = p0 + fp;
+    const bool fill = p < B;
+    float in[2] = {0.0f, 0.0f};  // the next step's input pair, loaded one step ahead; the latent pair
+    float aux = 0.0f;            // the current step's coefficient (latent) or target (stress row)
+    float aux_next = 0.0f;
+    if (is_z && fill) {
+      in[0] = w.z[(size_t)p * 6 + zk];
+      in[1] = w.z[(size_t)p * 6 + zk + 1];
+    }
+    auto load_inputs = [&](int t) {
+      if (!fill) return;
+      const size_t g = (size_t)t * B + p;
+      if (is_in) {
+        const float* src = fc < 6 ? w.strain + g * 6 + fc : w.rate + g * 6 + fc - 6;
+        in[0] = src[0];
+        in[1] = src[1];
+      } else if (is_z) {
+        aux_next = w.coef[g];
+      } else if (is_s && w.target) {
+        aux_next = w.target[g * 6 + srow];
+      }
+    };
+    load_inputs(0);
+    double sq = 0.0;
+    for (int t = 0;; ++t) {
+      if (t > 0 && fill) {  // finish step t - 1
+        if (is_z) {
+          in[0] = in[0] + aux * (S.y[6 + zk][fp] + bias_o[0]);
+          in[1] = in[1] + aux * (S.y[7 + zk][fp] + bias_o[1]);
+          float* zn = w.z + ((size_t)t * B + p) * 6 + zk;
+          zn[0] = in[0];
+          zn[1] = in[1];
+        } else if (is_s) {
+          const size_t g = (size_t)(t - 1) * B + p;
+          float s = S.y[srow][fp] + bias_o[0];
+          if (has_skip) {
+            float acc = 0.0f;
+#pragma unroll
+            for (int j = 0; j < 6; ++j)
+              acc += S.skip[6 * srow + j] * (S.e[(t - 1) & 1][fp][j] - S.z[(t - 1) & 1][fp][j]);
+            s += acc;
+          }
+          if (w.stress) w.stress[g * 6 + srow] = s;
+          if (w.target) {
+            const float d = s - aux;
+            sq += (double)d * d;
+            if (w.gS) w.gS[g * 6 + srow] = w.loss_scale * 2.0f * d;
+          }
+        }
+      }
+      if (t == T) break;
+      const size_t g0 = (size_t)t * B + p0, gq = (size_t)t * B + q0;
+      {  // input tile
+        const float v[2] = {is_in || is_z ? in[0] : 0.0f, is_in || is_z ? in[1] : 0.0f};
+        if (fc < 6) {
+          S.e[t & 1][fp][fc] = v[0];
+          S.e[t & 1][fp][fc + 1] = v[1];
+        } else if (is_z) {
+          S.z[t & 1][fp][zk] = v[0];
+          S.z[t & 1][fp][zk + 1] = v[1];
+        }
+        *reinterpret_cast<uint32_t*>(S.x + np_offset(fp, fc, XIN)) = pack_bf16(v[0], v[1]);
+        if (w.Xt && fill) {
+          __nv_bfloat16* xt = static_cast<__nv_bfloat16*>(w.Xt) + g0 + fp;
+          xt[(size_t)fc * R] = __float2bfloat16_rn(v[0]);
+          xt[(size_t)(fc + 1) * R] = __float2bfloat16_rn(v[1]);
+        }
+      }
+      aux = aux_next;
+      if (t + 1 < T) load_inputs(t + 1);
+#pragma unroll
+      for (int l = 0; l < 3; ++l) {
+        run = run && (l == 0 ? narrow_layer<XIN>(&S.bar, tmem, dw1, dx, phase, ok, nothing)
+                             : narrow_layer<HID>(&S.bar, tmem, l == 1 ? dw2 : dw3, dh, phase, ok, nothing));
+        if (!run) break;
+        float v[8];
+        tmem_ld8(taddr, v);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) v[c] += bias_l[l];
+        if (float* Zl = w.Z[l])
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+            if (c < count) Zl[(gq + c) * HID + unit] = v[c];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          v[c] = gelu(v[c]);
+          *reinterpret_cast<__nv_bfloat16*>(S.h + np_offset(8 * half + c, unit, HID)) = __float2bfloat16_rn(v[c]);
+        }
+        if (w.Ht[l]) {
+          __nv_bfloat16* row = static_cast<__nv_bfloat16*>(w.Ht[l]) + (size_t)unit * R;
+          store_row8(row, gq, v, count, (reinterpret_cast<uintptr_t>(row + gq) & 15u) == 0);
+        }
+      }
+      run = run && narrow_layer<HID>(&S.bar, tmem, dw4, dh, phase, ok, nothing);
+      if (!run) break;
+      if (quarter == 0) {
+        float v[8];
+        tmem_ld8(taddr, v);
+        if (lane < 12) {
+          float4* dst = reinterpret_cast<float4*>(&S.y[lane][8 * half]);
+          dst[0] = make_float4(v[0], v[1], v[2], v[3]);
+          dst[1] = make_float4(v[4], v[5], v[6], v[7]);
+        }
+      }
+      __syncthreads();  // S.y
+    }
+    // window loss of this tile: row tile % 8 of loss_part, whose remaining rows are zero
+    if (w.loss_part && run) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+      if (lane == 0) S.red[warp] = sq;
+      __syncthreads();
+      if (tid == 0) {
+        double tot = 0.0;
+        for (int i = 0; i < NW_THREADS / 32; ++i) tot += S.red[i];
+        const int wide = (B + TILE - 1) / TILE, col = tile / (TILE / NP), row = tile % (TILE / NP);
+        w.loss_part[(size_t)row * wide + col] = tot;
+        if (row == 0)
+          for (int r = 1; r < T; ++r)
+            if (r >= TILE / NP || col * (TILE / NP) + r >= ntiles) w.loss_part[(size_t)r * wide + col] = 0.0;
+      }
+    }
+    __syncthreads();  // the last step's S.y and S.red are read
+  }
+  if (__syncthreads_or(ok && run ? 0 : 1) && tid == 0 && w.err) atomicExch(w.err, 1u);
+  fence_before_sync();
+  __syncthreads();
+  if (warp == 0) {
+    fence_after_sync();
+    tmem_dealloc(tmem, 32);
+  }
+}
+
+// The thread of column 6 + k of the output-gradient tile keeps dz_k of its path.
+__global__ void __launch_bounds__(NW_THREADS, 1) rno_narrow_backward_kernel(const cib_rno_window w) {
+  extern __shared__ uint8_t smem_raw[];
+  NarrowBwdSmem& S = *reinterpret_cast<NarrowBwdSmem*>(smem_raw);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int quarter = warp & 3, half = warp >> 2;
+  const int unit = quarter * 32 + lane;
+  const int fp = tid & 15, fc = tid >> 4;  // path and column of the output-gradient tile
+  const int B = w.B, T = w.T;
+  const int ntiles = (B + NP - 1) / NP;
+  const size_t R = w.ldt > 0 ? (size_t)w.ldt : (size_t)B * T;
+
+  stage_matrix(S.w4t, static_cast<const __nv_bfloat16*>(w.Wt[3]), HID, YOUT, YOUT);
+  stage_matrix(S.w3t, static_cast<const __nv_bfloat16*>(w.Wt[2]), HID, HID, HID);
+  stage_matrix(S.w2t, static_cast<const __nv_bfloat16*>(w.Wt[1]), HID, HID, HID);
+  stage_matrix(S.w1t, static_cast<const __nv_bfloat16*>(w.Wt[0]), XIN, HID, HID);
+  zero_fill(S.w1t + XIN * HID * 2, (HID - XIN) * HID * 2);
+  for (int i = tid; i < 36; i += NW_THREADS) S.skip[i] = w.skip ? w.skip[i] : 0.0f;
+  if (warp == 0) tmem_alloc(&S.tmem, 32);
+  if (tid == 0) mbar_init(&S.bar, 1);
+  fence_smem_to_async();
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  const uint32_t tmem = S.tmem;
+  const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(8 * half);
+  const uint64_t dw4 = weight_desc(S.w4t, YOUT), dw3 = weight_desc(S.w3t, HID), dw2 = weight_desc(S.w2t, HID),
+                 dw1 = weight_desc(S.w1t, HID), ddy = tile_desc(S.dy, YOUT), dd = tile_desc(S.d, HID);
+  const bool has_skip = w.skip != nullptr;
+  const auto nothing = [] {};
+  const bool is_z = fc >= 6 && fc < 12;
+  __nv_bfloat16* dYt = static_cast<__nv_bfloat16*>(w.dYt);
+  uint32_t phase = 0;
+  bool ok = true, run = true;
+
+  for (int tile = blockIdx.x; tile < ntiles && run; tile += gridDim.x) {
+    const int p0 = tile * NP, q0 = p0 + 8 * half;
+    const int count = min(max(B - q0, 0), 8);
+    const bool fill = p0 + fp < B;
+    float dz = 0.0f;
+    float ng = 0.0f;  // loss gradient (columns 0..5) or coefficient (6..11) of the next (earlier) step
+    auto load_inputs = [&](int t) {
+      const size_t g = (size_t)t * B + p0 + fp;
+      ng = !fill ? 0.0f : fc < 6 ? w.gS[g * 6 + fc] : fc < 12 ? w.coef[g] : 0.0f;
+    };
+    load_inputs(T - 1);
+    float zv[8];  // pre-activations of this thread's unit, the layer that comes next
+    auto load_z = [&](int t, int l) {
+      const float* src = w.Z[l] + ((size_t)t * B + q0) * HID + unit;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) zv[c] = c < count ? src[c * HID] : 0.0f;
+    };
+    load_z(T - 1, 2);
+    for (int t = T - 1; t >= 0; --t) {
+      const size_t g0 = (size_t)t * B + p0, gq = (size_t)t * B + q0;
+      {
+        if (is_z && t < T - 1) {  // dz of the step after this one
+          float sk = 0.0f;
+          if (has_skip)
+#pragma unroll
+            for (int j = 0; j < 6; ++j) sk += S.skip[6 * j + fc - 6] * S.gs[(t + 1) & 1][fp][j];
+          dz = dz + S.dx[fc - 6][fp] - sk;
+        }
+        const float v = fc < 6 ? ng : is_z ? ng * dz : 0.0f;
+        if (fc < 6) S.gs[t & 1][fp][fc] = v;
+        const __nv_bfloat16 hv = __float2bfloat16_rn(v);
+        *reinterpret_cast<__nv_bfloat16*>(S.dy + np_offset(fp, fc, YOUT)) = hv;
+        if (fill) dYt[(size_t)fc * R + g0 + fp] = hv;
+      }
+      if (t > 0) load_inputs(t - 1);
+      // back through W_4, W_3, W_2 with the GELU derivative of Z_3, Z_2, Z_1; the derivative is
+      // evaluated while the tensor core works, the next layer's Z loads run beside it
+#pragma unroll
+      for (int l = 2; l >= 0; --l) {
+        float gg[8];
+        const auto derivative = [&] {
+#pragma unroll
+          for (int c = 0; c < 8; ++c) gg[c] = gelu_grad(zv[c]);
+          if (l > 0)
+            load_z(t, l - 1);
+          else if (t > 0)
+            load_z(t - 1, 2);
+        };
+        run = run && (l == 2 ? narrow_layer<YOUT>(&S.bar, tmem, dw4, ddy, phase, ok, derivative)
+                             : narrow_layer<HID>(&S.bar, tmem, l == 1 ? dw3 : dw2, dd, phase, ok, derivative));
+        if (!run) break;
+        float v[8];
+        tmem_ld8(taddr, v);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          v[c] = c < count ? bf16r(v[c] * gg[c]) : 0.0f;
+          *reinterpret_cast<__nv_bfloat16*>(S.d + np_offset(8 * half + c, unit, HID)) = __float2bfloat16_rn(v[c]);
+        }
+        __nv_bfloat16* row = static_cast<__nv_bfloat16*>(w.dZt[l]) + (size_t)unit * R;
+        store_row8(row, gq, v, count, (reinterpret_cast<uintptr_t>(row + gq) & 15u) == 0);
+      }
+      // dX = dZ_1 W_1: the latent rows 12..17 feed dz
+      run = run && narrow_layer<HID>(&S.bar, tmem, dw1, dd, phase, ok, nothing);
+      if (!run) break;
+      if (quarter == 0) {
+        float v[8];
+        tmem_ld8(taddr, v);
+        if (lane >= 12 && lane < 18) {
+          float4* dst = reinterpret_cast<float4*>(&S.dx[lane - 12][8 * half]);
+          dst[0] = make_float4(v[0], v[1], v[2], v[3]);
+          dst[1] = make_float4(v[4], v[5], v[6], v[7]);
+        }
+      }
+      __syncthreads();  // S.dx
+    }
+  }
+  if (__syncthreads_or(ok && run ? 0 : 1) && tid == 0 && w.err) atomicExch(w.err, 1u);
+  fence_before_sync();
+  __syncthreads();
+  if (warp == 0) {
+    fence_after_sync();
+    tmem_dealloc(tmem, 32);
+  }
+}
+
+// Whether a window runs on the narrow kernels: while its tiles of 16 paths run on every SM in at
+// most three turns.  Against the wide kernels: 512 paths x 50 steps forward 187 us (957),
+// backward 174 us (824); 4,736 paths x 20 steps (two turns) 153 us (402) and 148 us (354); in a
+// fourth turn (9,472 paths) the forward is at 296 us (404), but one inference step is slower,
+// 20.6 us (19.0; at 2,000 points 11.5 (19.0), at 5,000 16.9 (19.0)).
+bool narrow_window(int64_t B) { return (B + NP - 1) / NP <= 3 * (int64_t)sm_count(); }
+
 // The dynamic shared-memory limit is raised once per device and kernel (so that launches
 // recorded into a CUDA graph make no attribute call).
 int validate_common(const cib_rno_window* w) {
@@ -614,6 +1016,15 @@ extern "C" int cib_rno_window_forward(const cib_rno_window* w, void* stream) {
     rno_infer_kernel<<<igrid, RW_THREADS, ibytes, reinterpret_cast<cudaStream_t>(stream)>>>(*w);
     return check_launch();
   }
+  // (its loss grouping needs 8 rows of loss_part)
+  if (narrow_window(w->B) && (!w->loss_part || w->T >= TILE / NP)) {
+    const size_t nbytes = sizeof(NarrowFwdSmem);
+    if (allow_dynamic_smem(reinterpret_cast<const void*>(rno_narrow_forward_kernel), (int)nbytes) != CIB_OK)
+      return CIB_ECUDA;
+    const unsigned ngrid = (unsigned)std::min<int64_t>((w->B + NP - 1) / NP, sm_count());
+    rno_narrow_forward_kernel<<<ngrid, NW_THREADS, nbytes, reinterpret_cast<cudaStream_t>(stream)>>>(*w);
+    return check_launch();
+  }
   const size_t bytes = sizeof(FwdSmem);
   if (allow_dynamic_smem(reinterpret_cast<const void*>(rno_window_forward_kernel), (int)bytes) != CIB_OK)
     return CIB_ECUDA;
@@ -631,6 +1042,14 @@ extern "C" int cib_rno_window_backward(const cib_rno_window* w, void* stream) {
     if (!w->Z[l] || !aligned16(w->Z[l]) || !w->dZt[l]) return CIB_EINVAL;
   if (!w->gS || !w->dYt) return CIB_EINVAL;
   if (w->B == 0) return CIB_OK;
+  if (narrow_window(w->B)) {
+    const size_t nbytes = sizeof(NarrowBwdSmem);
+    if (allow_dynamic_smem(reinterpret_cast<const void*>(rno_narrow_backward_kernel), (int)nbytes) != CIB_OK)
+      return CIB_ECUDA;
+    const unsigned ngrid = (unsigned)std::min<int64_t>((w->B + NP - 1) / NP, sm_count());
+    rno_narrow_backward_kernel<<<ngrid, NW_THREADS, nbytes, reinterpret_cast<cudaStream_t>(stream)>>>(*w);
+    return check_launch();
+  }
   const size_t bytes = sizeof(BwdSmem);
   if (allow_dynamic_smem(reinterpret_cast<const void*>(rno_window_backward_kernel), (int)bytes) != CIB_OK)
     return CIB_ECUDA;

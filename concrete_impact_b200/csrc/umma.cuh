@@ -46,18 +46,26 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
 
-// Waits for the phase with the given parity; false after WAIT_LIMIT_NS.
+__device__ __forceinline__ bool mbar_try(uint32_t a, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(done)
+      : "r"(a), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+
+// Waits for the phase with the given parity; false after WAIT_LIMIT_NS.  The clock is read only
+// when a wait lasts: a layer's wait is shorter than a read of the global timer is slow.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   const uint32_t a = smem_u32(bar);
+#pragma unroll 1
+  for (int i = 0; i < 32; ++i)
+    if (mbar_try(a, parity)) return true;
   const uint64_t t0 = now_ns();
   while (true) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (done) return true;
+    if (mbar_try(a, parity)) return true;
     if (now_ns() - t0 > WAIT_LIMIT_NS) return false;
   }
 }
@@ -94,6 +102,35 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem, uint32_t a_base, uint32_
   }
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
+}
+
+// The same from descriptors of the operands' first K = 16 step; the next steps start A_STEP and
+// B_STEP bytes further (unrolled: the issue is on the critical path of a short layer).
+template <int K, int A_STEP, int B_STEP>
+__device__ __forceinline__ void mma_bf16_steps(uint32_t tmem, uint64_t da, uint64_t db, int n, uint64_t* bar) {
+  const uint32_t idesc = idesc_bf16(n);
+#pragma unroll
+  for (int s = 0; s < K / 16; ++s) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n}\n" ::"r"(tmem),
+        "l"(da + (uint64_t)(s * (A_STEP >> 4))), "l"(db + (uint64_t)(s * (B_STEP >> 4))), "r"(idesc),
+        "r"(s > 0 ? 1u : 0u), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
+        : "memory");
+  }
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
+               : "memory");
+}
+
+// 8 consecutive fp32 columns of this thread's TMEM lane.
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
+  uint32_t r[8];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[j]);
 }
 
 // 16 consecutive fp32 columns of this thread's TMEM lane (warp w reads lanes 32 (w % 4) ..).

@@ -519,6 +519,29 @@ typedef struct cib_rno_window {
 int cib_rno_window_forward(const cib_rno_window* w, void* stream);
 int cib_rno_window_backward(const cib_rno_window* w, void* stream);
 
+/* Weight and bias gradients of the four layers from a window's transposed buffers:
+ * gw[l] (M x N) = A[l] B[l]^T and gb[l] (M) = row sums of A[l] over K columns (a multiple of
+ * 16; ld, a multiple of 8, is the leading dimension of all of them), bf16 operands with fp32
+ * accumulation, split over at most `splits` K slices added in order.  M <= 128, N a multiple of
+ * 16 up to 128.  Work space: partial (splits x sum of M N floats, 16-byte aligned) and
+ * row_partial (splits x 512 doubles).  The gradients of the reference's autograd training step
+ * (src/concrete_impact/nn/training/rve_rno.py:200-415). */
+typedef struct cib_rno_wgrad {
+  int32_t K;
+  int32_t splits;
+  int64_t ld;
+  int32_t M[4];
+  int32_t N[4];
+  const void* A[4];
+  const void* B[4];
+  float* gw[4];
+  float* gb[4];
+  float* partial;
+  double* row_partial;
+  unsigned int* err;
+} cib_rno_wgrad;
+int cib_rno_weight_gradients(const cib_rno_wgrad* g, void* stream);
+
 /* --- Explicit macro dynamics (FE^2)---------------------------------------------------
  * Velocity-Verlet step of src/fem/dynamics/material.py:164-219 with a lumped mass and
  * homogeneous Dirichlet DOFs (fixed[i] != 0): predictor u' = u + dt v + dt^2/2 a, then
