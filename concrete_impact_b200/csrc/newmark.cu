@@ -12,18 +12,21 @@
 //     reference's sparse direct solve (src/fem/solvers/linear.py:15).
 //
 // CSR rows are handled one warp per row (a Hex8 row has at most 81 entries, so the lanes
-// read contiguous values and column indices).  The CG runs as three kernels per iteration
+// read contiguous values and column indices).  Systems of up to 28,416 rows whose share of
+// the matrix fits an SM's shared memory run the CG as one persistent launch (csr_pcg_grid.cu);
+// beyond that it runs as three kernels per iteration
 // (matrix product + p.q partials; x, r, z update + r.z and r.r partials; new direction).
 // Every dot product is reduced in a fixed order: one partial per block, then each block
 // of the next kernel sums all partials in the same order, so every block holds the same
 // scalar and results are bitwise repeatable.  The iteration count is bounded by `maxit`;
 // the host reads the device status every `check_every` iterations, and kernels launched
-// after convergence return at once.  Nothing waits on another block.
+// after convergence return at once.  Nothing here waits on another block.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
 
 #include "cib_common.cuh"
+#include "csr_pcg_grid.cuh"
 
 namespace cib {
 namespace {
@@ -43,6 +46,10 @@ constexpr int ST_REL = ST + 2;                  //   ||r|| / ||b||
 constexpr int ST_BNORM = ST + 3;                //   ||b|| (free DOFs)
 constexpr int ST_RZ = ST + 4;                   //   r.z of the current direction, two slots
 static_assert(ST_RZ + 2 <= CIB_CSR_PCG_WORK_DOUBLES, "work layout");
+static_assert(pcg_grid_out(1) <= CIB_CSR_PCG_WORK_DOUBLES, "work layout of the persistent solve");
+constexpr int BLOCK_PART = pcg_grid_part(PCG_BLOCK_RHS);  // block solve: then the results
+static_assert(BLOCK_PART + pcg_grid_out(PCG_BLOCK_RHS) <= CIB_CSR_PCG_BLOCK_WORK_DOUBLES(0), "work layout of the block solve");
+static_assert(CIB_CSR_PCG_WORK_DOUBLES <= CIB_CSR_PCG_BLOCK_WORK_DOUBLES(0), "six single solves in its place");
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -326,15 +333,17 @@ extern "C" int cib_csr_spmv(int64_t n, const int64_t* indptr, const int64_t* ind
   return check_launch();
 }
 
-extern "C" int cib_csr_pcg(int64_t n, const int64_t* indptr, const int64_t* indices, const double* values,
-                           const uint8_t* free_mask, const double* dinv, const double* b, double* x, double* r,
-                           double* z, double* p, double* q, double* work, double rtol, int32_t maxit,
-                           int32_t check_every, int32_t* status, int32_t* iterations, double* relative_residual,
-                           void* stream) {
-  if (n <= 0 || !indptr || !indices || !values || !free_mask || !dinv || !b || !x || !r || !z || !p || !q || !work ||
-      !status || !iterations || !relative_residual || maxit < 0 || check_every <= 0 || !(rtol >= 0.0))
-    return CIB_EINVAL;
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+namespace cib {
+namespace {
+
+// A launch per phase, the host reading the status every `check_every` iterations.
+int csr_pcg_launches(const CsrSystem& a, const double* b, double* x, double* r, double* z, double* p, double* q,
+                     double* work, double rtol, int32_t maxit, int32_t check_every, int32_t* status,
+                     int32_t* iterations, double* relative_residual, cudaStream_t st) {
+  const int64_t n = a.n;
+  const int64_t *indptr = a.indptr, *indices = a.indices;
+  const double *values = a.values, *dinv = a.dinv;
+  const uint8_t* free_mask = a.free_mask;
   const int g_rows = rows_grid(n), g_vec = vec_grid(n);
   if (g_rows > PCG_MAX_GRID || g_vec > PCG_MAX_GRID) return CIB_ERANGE;
   pcg_init_kernel<<<g_vec, NM_THREADS, 0, st>>>(n, free_mask, dinv, b, x, r, z, p, work);
@@ -360,4 +369,45 @@ extern "C" int cib_csr_pcg(int64_t n, const int64_t* indptr, const int64_t* indi
   *iterations = (int32_t)host[1];
   *relative_residual = host[2];
   return CIB_OK;
+}
+
+}  // namespace
+}  // namespace cib
+
+extern "C" int cib_csr_pcg(int64_t n, const int64_t* indptr, const int64_t* indices, const double* values,
+                           const uint8_t* free_mask, const double* dinv, const double* b, double* x, double* r,
+                           double* z, double* p, double* q, double* work, double rtol, int32_t maxit,
+                           int32_t check_every, int32_t* status, int32_t* iterations, double* relative_residual,
+                           void* stream) {
+  if (n <= 0 || !indptr || !indices || !values || !free_mask || !dinv || !b || !x || !r || !z || !p || !q || !work ||
+      !status || !iterations || !relative_residual || maxit < 0 || check_every <= 0 || !(rtol >= 0.0))
+    return CIB_EINVAL;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const CsrSystem a{n, indptr, indices, values, free_mask, dinv};
+  const PcgGridWork w{z, r, p, work};
+  const int rc = csr_pcg_grid(a, 1, b, x, w, rtol, maxit, status, iterations, relative_residual, st);
+  if (rc != CIB_ERANGE) return rc;
+  return csr_pcg_launches(a, b, x, r, z, p, q, work, rtol, maxit, check_every, status, iterations, relative_residual, st);
+}
+
+extern "C" int cib_csr_pcg_block(int64_t n, const int64_t* indptr, const int64_t* indices, const double* values,
+                                 const uint8_t* free_mask, const double* dinv, const double* b, double* x,
+                                 double* work, double rtol, int32_t maxit, int32_t check_every, int32_t* status,
+                                 int32_t* iterations, double* relative_residual, void* stream) {
+  if (n <= 0 || !indptr || !indices || !values || !free_mask || !dinv || !b || !x || !work || !status || !iterations ||
+      !relative_residual || maxit < 0 || check_every <= 0 || !(rtol >= 0.0))
+    return CIB_EINVAL;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const CsrSystem a{n, indptr, indices, values, free_mask, dinv};
+  double* vectors = work + CIB_CSR_PCG_BLOCK_WORK_DOUBLES(0);  // 12 n
+  const PcgGridWork w{vectors, vectors + PCG_BLOCK_RHS * n, work, work + BLOCK_PART};
+  int rc = csr_pcg_grid(a, PCG_BLOCK_RHS, b, x, w, rtol, maxit, status, iterations, relative_residual, st);
+  for (int j = 0; rc == CIB_ERANGE && j < PCG_BLOCK_RHS; ++j) {
+    rc = cib_csr_pcg(n, indptr, indices, values, free_mask, dinv, b + j * n, x + j * n, vectors, vectors + n,
+                     vectors + 2 * n, vectors + 3 * n, work, rtol, maxit, check_every, status + j, iterations + j,
+                     relative_residual + j, stream);
+    if (rc != CIB_OK) return rc;
+    rc = CIB_ERANGE;
+  }
+  return rc == CIB_ERANGE ? CIB_OK : rc;
 }

@@ -70,6 +70,7 @@ class _ReducedSystem:
         self.free = torch.ones(n, dtype=torch.uint8, device=device)
         self.r, self.z, self.p, self.q = (torch.empty(n, **f64) for _ in range(4))
         self.work = torch.zeros(CSR_PCG_WORK_DOUBLES, **f64)
+        self.block_work: torch.Tensor | None = None  # CIB_CSR_PCG_BLOCK_WORK_DOUBLES(n), with the first tangent
         self.rtol, self.maxit = relative_tolerance, max_iterations
         self.device = device
         self.iterations = 0
@@ -92,6 +93,23 @@ class _ReducedSystem:
                                       _native.stream_ptr()), "cib_csr_pcg")  # fmt: skip
         self.iterations += int(iterations.value)
         return x, int(status.value), int(iterations.value), float(rel.value)
+
+    def solve_six(self, lib, rhs: torch.Tensor) -> tuple[torch.Tensor, list[int]]:
+        """x (6, n) and the status of each row of rhs (6, n), in one pass over the matrix."""
+        if not rhs.is_cuda:  # a host stand-in of the device has the single solve only
+            rows = [self.solve(lib, b) for b in rhs]
+            return torch.stack([x for x, _, _, _ in rows]), [status for _, status, _, _ in rows]
+        if self.block_work is None:
+            self.block_work = torch.empty(12 * self.n + 24576, dtype=torch.float64, device=self.device)
+        x = torch.empty((6, self.n), dtype=torch.float64, device=self.device)
+        status, iterations, rel = (ctypes.c_int32 * 6)(), (ctypes.c_int32 * 6)(), (ctypes.c_double * 6)()
+        _native.check(lib.cib_csr_pcg_block(self.n, self.indptr.data_ptr(), self.indices.data_ptr(),
+                                            self.values.data_ptr(), self.free.data_ptr(), self.dinv.data_ptr(),
+                                            rhs.contiguous().data_ptr(), x.data_ptr(), self.block_work.data_ptr(),
+                                            float(self.rtol), int(self.maxit), 16, status, iterations, rel,
+                                            _native.stream_ptr()), "cib_csr_pcg_block")  # fmt: skip
+        self.iterations += sum(iterations)
+        return x, list(status)
 
 
 class GeneralRVEOperators:
@@ -251,13 +269,10 @@ def effective_tangent(ops: GeneralRVEOperators, tangent) -> torch.Tensor:
         return k_ee / ops.volume
     k_we = torch.stack([ops.Tt.mv(lib, ka[j]) for j in range(6)])  # (6, m)
     ops.reduced.prepare(lib, ops.gather_reduced(tangent.values()))
-    sens = []
-    for j in range(6):
-        x, status, _, _ = ops.reduced.solve(lib, k_we[j])
-        if status != 0 or not bool(torch.isfinite(x).all()):
-            raise RVEEquilibriumError("non_finite_effective_tangent_sensitivity", {"reduced_dof_count": ops.m})
-        sens.append(x)
-    return (k_ee - k_we @ torch.stack(sens).T) / ops.volume
+    sens, status = ops.reduced.solve_six(lib, k_we)
+    if any(status) or not bool(torch.isfinite(sens).all()):
+        raise RVEEquilibriumError("non_finite_effective_tangent_sensitivity", {"reduced_dof_count": ops.m})
+    return (k_ee - k_we @ sens.T) / ops.volume
 
 
 def _general_response(model, request, committed, macro, w, u, asm, iterations, backtracks, rn, tol, ops, io):

@@ -587,8 +587,9 @@ int cib_csr_spmv(int64_t n, const int64_t* indptr, const int64_t* indices, const
  * n-vectors of scratch, work CIB_CSR_PCG_WORK_DOUBLES doubles (device).  Stops when
  * ||r|| <= rtol ||b|| or after maxit iterations; the host reads the device status every
  * check_every iterations.  Host outputs: status 0 converged, 1 iteration limit, 2 breakdown
- * (p.Ap <= 0 or a non-finite value); iterations; relative_residual ||r|| / ||b||.  The dot
- * products are reduced in a fixed order: bitwise repeatable.  Returns CIB_ERANGE when n
+ * (p.Ap <= 0 or a non-finite value); iterations; relative_residual ||r|| / ||b||.  Up to
+ * 28,416 rows the solve is one cooperative launch, read once at its end (check_every then has
+ * no effect).  The dot products are reduced in a fixed order: bitwise repeatable.  Returns CIB_ERANGE when n
  * needs more than CIB_CSR_PCG_MAX_GRID blocks of partials. */
 #define CIB_CSR_PCG_MAX_GRID 1024
 #define CIB_CSR_PCG_WORK_DOUBLES (3 * CIB_CSR_PCG_MAX_GRID + 8)
@@ -596,6 +597,15 @@ int cib_csr_pcg(int64_t n, const int64_t* indptr, const int64_t* indices, const 
                 const uint8_t* free_mask, const double* dinv, const double* b, double* x, double* r, double* z,
                 double* p, double* q, double* work, double rtol, int32_t maxit, int32_t check_every, int32_t* status,
                 int32_t* iterations, double* relative_residual, void* stream);
+
+/* Six right-hand sides of one matrix (rows of b and x, 6 x n): as six calls of cib_csr_pcg, in
+ * one pass over the matrix where that takes the system.  status, iterations and
+ * relative_residual hold six entries; work CIB_CSR_PCG_BLOCK_WORK_DOUBLES(n) doubles. */
+#define CIB_CSR_PCG_BLOCK_WORK_DOUBLES(n) (12 * (n) + 24576)
+int cib_csr_pcg_block(int64_t n, const int64_t* indptr, const int64_t* indices, const double* values,
+                      const uint8_t* free_mask, const double* dinv, const double* b, double* x, double* work,
+                      double rtol, int32_t maxit, int32_t check_every, int32_t* status, int32_t* iterations,
+                      double* relative_residual, void* stream);
 
 /* --- Energy-based RVE-RNO (the reference's surrogate family) ------------------------------
  * FP32 update of src/concrete_impact/nn/models/rve_rno.py:334-418 (EnergyDissipationRVERNO,
