@@ -69,6 +69,15 @@ class MaterialAssemblyCache:
     _host: dict = field(default_factory=dict, repr=False, compare=False)
 
     @property
+    def csr_pattern(self) -> tuple[torch.Tensor, torch.Tensor]:
+        """csr_indptr and csr_indices on the device, copied once; results share them on any stream."""
+        if "csr" not in self._host:
+            self._host["csr"] = tuple(torch.as_tensor(a, device=self.grads.device) for a in (self.csr_indptr, self.csr_indices))
+        for t in self._host["csr"]:
+            t.record_stream(torch.cuda.current_stream(t.device))
+        return self._host["csr"]
+
+    @property
     def jacobian_weights(self) -> np.ndarray:
         """(E, 8) det J times the Gauss weight."""
         if "jw" not in self._host:
@@ -214,9 +223,8 @@ def assemble_hex8_material_response_cached(nodes, elements, material, committed_
             # (and its notices that CSR support is beta and the check is off)
             with warnings.catch_warnings():
                 warnings.simplefilter("ignore", UserWarning)
-                tangent = torch.sparse_csr_tensor(torch.as_tensor(cache.csr_indptr, device=dev),
-                                                  torch.as_tensor(cache.csr_indices, device=dev), values,
-                                                  size=(n_dof, n_dof), check_invariants=False)  # fmt: skip
+                tangent = torch.sparse_csr_tensor(*cache.csr_pattern, values, size=(n_dof, n_dof),
+                                                  check_invariants=False)
     else:
         tangent = csr_matrix((n_dof, n_dof)) if io.host else None
     return NonlinearSolidAssemblyResult(

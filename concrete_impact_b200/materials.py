@@ -21,7 +21,7 @@ from __future__ import annotations
 import ctypes
 import math
 from dataclasses import dataclass, field
-from typing import Any, Protocol
+from typing import Any, NamedTuple, Protocol
 
 import numpy as np
 import torch
@@ -183,9 +183,7 @@ def _require_six_component_strains(strains: Any) -> Any:
 
 def _new_flags(device: torch.device) -> torch.Tensor:
     """[first_failure (all bits set = none), active_count] as int64 on the device."""
-    flags = torch.zeros(2, dtype=torch.int64, device=device)
-    flags[0] = -1
-    return flags
+    return torch.arange(-1, 1, dtype=torch.int64, device=device)
 
 
 # --------------------------------------------------------------------------------------
@@ -313,11 +311,10 @@ def j2vp_update_points(
     variables["viscoplastic_multiplier"] = io.out(vpm1)
     diagnostics: dict[str, Any] = {}
     if n > 0:
-        names = _native.j2_diagnostic_names()
-        keep = [i for i, name in enumerate(names) if _keep_j2_diagnostic(name, active, rate is not None)]
-        rows = io.out(diag[keep])
-        for slot, i in enumerate(keep):
-            diagnostics[names[i]] = rows[slot]
+        rows = io.out(diag)
+        for i, name in enumerate(_native.j2_diagnostic_names()):
+            if _keep_j2_diagnostic(name, active, rate is not None):
+                diagnostics[name] = rows[i]
     return MaterialPointResponse(
         stresses=io.out(stress),
         state=MaterialState(variables),
@@ -519,6 +516,12 @@ class RVEPhase:
     material: MaterialModel
 
 
+class _Everywhere(NamedTuple):
+    """A diagnostic with one value at all points of a phase."""
+
+    value: float
+
+
 @dataclass(frozen=True)
 class PhasedMaterialModel:
     """Dispatch fixed integration-point subsets to phase material models."""
@@ -563,22 +566,24 @@ class PhasedMaterialModel:
         io = _Io(strains)
         eps = io.to_device(strains, (point_count, component_count))
         rates = None if request.strain_rates is None else io.to_device(request.strain_rates, eps.shape)
-        stresses = torch.zeros_like(eps)
-        tangents = (
-            torch.zeros((point_count, component_count, component_count), dtype=torch.float64, device=io.device)
-            if requirements.tangent
-            else None
-        )
-        free_energy = torch.zeros(point_count, dtype=torch.float64, device=io.device) if requirements.free_energy else None
-        dissipation = torch.zeros(point_count, dtype=torch.float64, device=io.device) if requirements.dissipation else None
+        ids_of = [np.flatnonzero(phase_ids == phase_id) for phase_id in range(len(self.phases))]
+        new = torch.empty if sum(ids.size for ids in ids_of) == point_count else torch.zeros  # points of no phase: zeros
+        where = dict(dtype=torch.float64, device=io.device)
+        stresses = new(eps.shape, **where)
+        tangents = new((point_count, component_count, component_count), **where) if requirements.tangent else None
+        free_energy = new(point_count, **where) if requirements.free_energy else None
+        dissipation = new(point_count, **where) if requirements.dissipation else None
         next_variables: dict[str, Any] = {}
-        phase_diagnostics: list[tuple[torch.Tensor, dict[str, Any]]] = []
-        for phase_id, phase in enumerate(self.phases):
-            ids = torch.as_tensor(np.flatnonzero(phase_ids == phase_id), device=io.device)
+        results: list[tuple[torch.Tensor, list, dict[str, Any]]] = []
+        for phase, phase_points in zip(self.phases, ids_of):
+            ids = torch.as_tensor(phase_points, device=io.device)
             phase_state = _decode_phase_state(state, phase.name)
+            inputs = [None if a is None else io.empty(ids.numel(), component_count) for a in (eps, rates)]
+            _native.copy_rows(ids, [(a, to, component_count, 0.0) for a, to in zip((eps, rates), inputs) if a is not None],
+                              scatter=False)  # fmt: skip
             phase_request = MaterialPointRequest(
-                strains=eps.index_select(0, ids),
-                strain_rates=None if rates is None else rates.index_select(0, ids),
+                strains=inputs[0],
+                strain_rates=inputs[1],
                 time_step=request.time_step,
                 kinematics=request.kinematics,
                 update_settings=request.update_settings,
@@ -593,31 +598,39 @@ class PhasedMaterialModel:
                 )
                 diagnostics = dict(response.diagnostics)
                 diagnostics.update(extra)
-                diagnostics["viscoplastic_active"] = torch.zeros(ids.numel(), dtype=torch.float64, device=io.device)
+                diagnostics["viscoplastic_active"] = _Everywhere(0.0)
             else:
                 response = phase.material.update(phase_request, device_state, requirements)
                 diagnostics = dict(response.diagnostics)
-            stresses.index_copy_(0, ids, response.stresses)
-            if tangents is not None:
-                if response.tangents is None:
-                    raise ValueError("Phased material requested a tangent but received None.")
-                tangents.index_copy_(0, ids, response.tangents)
-            if free_energy is not None:
-                if response.free_energy is None:
-                    raise ValueError("Phased material requested free energy but received None.")
-                free_energy.index_copy_(0, ids, response.free_energy)
-            if dissipation is not None:
-                if response.dissipation is None:
-                    raise ValueError("Phased material requested dissipation but received None.")
-                dissipation.index_copy_(0, ids, response.dissipation)
+            fields = [(stresses, response.stresses)]
+            for name, to, value in (("a tangent", tangents, response.tangents),
+                                    ("free energy", free_energy, response.free_energy),
+                                    ("dissipation", dissipation, response.dissipation)):  # fmt: skip
+                if to is not None:
+                    if value is None:
+                        raise ValueError(f"Phased material requested {name} but received None.")
+                    fields.append((to, value))
             for name, values in response.state.variables.items():
                 next_variables[encode_phase_state_key(phase.name, name)] = io.out(values)
-            phase_diagnostics.append((ids, diagnostics))
-        names = sorted(set().union(*(d.keys() for _, d in phase_diagnostics)))
-        combined = {name: torch.full((point_count,), float("nan"), dtype=torch.float64, device=io.device) for name in names}
-        for ids, diagnostics in phase_diagnostics:
-            for name, values in diagnostics.items():
-                combined[name].index_copy_(0, ids, io.to_device(values))
+            results.append((ids, fields, diagnostics))
+        names = sorted(set().union(*(d.keys() for _, _, d in results)))
+        missing = _Everywhere(float("nan"))
+        block = torch.full((len(names), point_count), missing.value, **where) if new is torch.zeros else io.empty(len(names), point_count)
+        combined = dict(zip(names, block))
+        for ids, fields, diagnostics in results:
+            copies = []
+            for name, to in combined.items():
+                values = diagnostics.get(name, missing)
+                if isinstance(values, _Everywhere):
+                    copies.append((None, to, 1, values.value))
+                else:
+                    fields.append((to, io.to_device(values)))
+            for to, values in fields:
+                if values.shape == (ids.numel(), *to.shape[1:]) and values.dtype == torch.float64 and values.is_cuda:
+                    copies.append((values.contiguous(), to, math.prod(to.shape[1:]), 0.0))
+                else:
+                    to.index_copy_(0, ids, values)
+            _native.copy_rows(ids, copies, scatter=True)
         return MaterialPointResponse(
             stresses=io.out(stresses),
             state=MaterialState(next_variables),

@@ -598,6 +598,19 @@ int cib_csr_pcg(int64_t n, const int64_t* indptr, const int64_t* indices, const 
                 double* p, double* q, double* work, double rtol, int32_t maxit, int32_t check_every, int32_t* status,
                 int32_t* iterations, double* relative_residual, void* stream);
 
+/* Rows of several FP64 arrays gathered (dst[i] = src[ids[i]], scatter 0) or scattered
+ * (dst[ids[i]] = src[i], or `fill` where src is NULL) for i < count, in one launch: at most
+ * CIB_ROW_COPIES arrays, read from host memory.  ids are distinct. */
+#define CIB_ROW_COPIES 32
+typedef struct cib_row_copy {
+  const double* src;
+  double* dst;
+  int64_t width;
+  double fill;
+} cib_row_copy;
+int cib_copy_rows(int64_t count, const int64_t* ids, int32_t arrays, const cib_row_copy* copies, int32_t scatter,
+                  void* stream);
+
 /* Six right-hand sides of one matrix (rows of b and x, 6 x n): as six calls of cib_csr_pcg, in
  * one pass over the matrix where that takes the system.  status, iterations and
  * relative_residual hold six entries; work CIB_CSR_PCG_BLOCK_WORK_DOUBLES(n) doubles. */
