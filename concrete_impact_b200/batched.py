@@ -27,9 +27,7 @@ _KIND_D2H = 2
 
 
 def _flags(device: torch.device) -> torch.Tensor:
-    flags = torch.zeros(2, dtype=torch.int64, device=device)
-    flags[0] = -1
-    return flags
+    return torch.arange(-1, 1, dtype=torch.int64, device=device)
 
 
 @dataclass
