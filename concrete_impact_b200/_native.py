@@ -245,6 +245,7 @@ SIGNATURES: dict[str, tuple[object, list[object]]] = {
                       + [_P, _P, ctypes.c_int32, _P, ctypes.c_int32, _P]),
     "cib_counter_increment": (_I, [_P, _P]),
     "cib_rno_window_forward": (_I, [_P, _P]),
+    "cib_rno_predict": (_I, [_P, _P, _P]),
     "cib_rno_window_backward": (_I, [_P, _P]),
     "cib_rno_weight_gradients": (_I, [_P, _P]),
     "cib_rno_gate_prepare": (_I, [_I64, _P, _P, _D, _D, _P, _D] + [_P] * 7),
@@ -346,6 +347,14 @@ def _j2_diagnostic_names() -> tuple[str, ...]:
 def j2_diagnostic_names() -> list[str]:
     """Names of the diagnostic rows written by ``cib_j2vp_update``, in row order."""
     return list(_j2_diagnostic_names())
+
+
+class RNOPredictInputsC(ctypes.Structure):
+    """``cib_rno_predict_inputs``."""
+
+    _fields_ = [("strain", ctypes.c_void_p), ("rate", ctypes.c_void_p), ("z", ctypes.c_void_p), ("stress", ctypes.c_void_p),
+                ("strain_scale", ctypes.c_double), ("rate_scale", ctypes.c_double), ("stress_scale", ctypes.c_double),
+                ("strain_f64", ctypes.c_int32), ("rate_f64", ctypes.c_int32)]  # fmt: skip
 
 
 class RowCopyC(ctypes.Structure):

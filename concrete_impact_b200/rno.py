@@ -520,20 +520,36 @@ class RNOSurrogate:
             buffers = {"M": M, "z": torch.empty((2, M, 6), dtype=torch.float32, device=dev),
                        "stress": torch.empty((1, M, 6), dtype=torch.float32, device=dev)}  # fmt: skip
         s = self.scales
-        sn = (strain / s.strain).float().contiguous()
-        rn = (rate / s.rate).float().contiguous()
         cf = coef.float().contiguous()
-        buffers["z"][0].copy_(z)
         c = _native.RNOWindowC()
         c.B, c.T, c.hidden = M, 1, self.config.hidden
-        c.strain, c.rate, c.coef, c.z = sn.data_ptr(), rn.data_ptr(), cf.data_ptr(), buffers["z"].data_ptr()
+        c.coef, c.z = cf.data_ptr(), buffers["z"].data_ptr()
         for i, L in enumerate(self.layers):
             c.W[i], c.bias[i] = L.wb.data_ptr(), L.b.data_ptr()
         c.skip = None if self.skip is None else self.skip.data_ptr()
         c.stress = buffers["stress"].data_ptr()
         c.err = self.err.data_ptr()
+        if self._raw_inputs(strain, rate, z, M):
+            scratch = torch.empty((2, M, 6), dtype=torch.float32, device=dev)
+            out = torch.empty((M, 6), dtype=torch.float32, device=dev)
+            c.strain, c.rate = scratch[0].data_ptr(), scratch[1].data_ptr()
+            x = _native.RNOPredictInputsC(strain.data_ptr(), rate.data_ptr(), z.data_ptr(), out.data_ptr(), s.strain,
+                                          s.rate, s.stress, strain.dtype == torch.float64, rate.dtype == torch.float64)  # fmt: skip
+            _check(self.lib.cib_rno_predict(ctypes.byref(c), ctypes.byref(x), _native.stream_ptr()), "cib_rno_predict")
+            return out, buffers["z"][1], buffers
+        sn = (strain / s.strain).float().contiguous()
+        rn = (rate / s.rate).float().contiguous()
+        buffers["z"][0].copy_(z)
+        c.strain, c.rate = sn.data_ptr(), rn.data_ptr()
         _check(self.lib.cib_rno_window_forward(ctypes.byref(c), _native.stream_ptr()), "cib_rno_window_forward")
         return buffers["stress"][0] * s.stress, buffers["z"][1], buffers
+
+    def _raw_inputs(self, strain: torch.Tensor, rate: torch.Tensor, z: torch.Tensor, M: int) -> bool:
+        """Whether the step can take its inputs as they are: contiguous (M, 6) on the device,
+        strain and rate FP32 or FP64, the latent state FP32.  Anything else goes through torch."""
+        kinds = ((strain, (torch.float32, torch.float64)), (rate, (torch.float32, torch.float64)), (z, (torch.float32,)))
+        return M > 0 and all(t.shape == (M, 6) and t.is_cuda and t.is_contiguous() and t.dtype in kind and not t.requires_grad
+                             for t, kind in kinds)  # fmt: skip
 
     def predict_normalized(self, strain_n: torch.Tensor, rate_n: torch.Tensor, coef: torch.Tensor, z: torch.Tensor,
                            stress_n: torch.Tensor) -> None:  # fmt: skip

@@ -517,6 +517,23 @@ typedef struct cib_rno_window {
   unsigned int* err;
 } cib_rno_window;
 int cib_rno_window_forward(const cib_rno_window* w, void* stream);
+
+/* One step (w->T = 1) from physical inputs: strain and rate (B, 6), each FP64 or FP32, are
+ * divided by their scales into the buffers w->strain and w->rate, the latent state z (B, 6) is
+ * copied to w->z[0] (z may be any part of w->z), and stress (B, 6) receives the stress times
+ * stress_scale. */
+typedef struct cib_rno_predict_inputs {
+  const void* strain;
+  const void* rate;
+  const float* z;
+  float* stress;
+  double strain_scale;
+  double rate_scale;
+  double stress_scale;
+  int32_t strain_f64;
+  int32_t rate_f64;
+} cib_rno_predict_inputs;
+int cib_rno_predict(const cib_rno_window* w, const cib_rno_predict_inputs* in, void* stream);
 int cib_rno_window_backward(const cib_rno_window* w, void* stream);
 
 /* Weight and bias gradients of the four layers from a window's transposed buffers:
