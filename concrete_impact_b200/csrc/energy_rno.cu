@@ -22,6 +22,7 @@
 #include <stdint.h>
 
 #include "cib_common.cuh"
+#include "f32x2.cuh"
 
 namespace cib {
 namespace {
@@ -462,25 +463,6 @@ __device__ __forceinline__ float silu_fast(float z, float d, float& q) {
   q = fmaf(r, fmaf(-d, r, 1.0f), r);
   const float h = z * q;
   return fmaf(fmaf(-h, d, z), q, h);
-}
-
-// Two single-precision multiply-adds in one instruction, each rounded as fmaf rounds it.
-using f32x2 = unsigned long long;
-
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ float2 unpack2(f32x2 v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
 }
 
 // C consecutive floats of a row of shared memory, at a multiple of C from an aligned start.

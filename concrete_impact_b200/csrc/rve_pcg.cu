@@ -498,7 +498,7 @@ struct Solver {
       T* y = ye + e;
       auto out = [&](int aa, int dd, T v) { y[(3 * aa + dd) * es] = v; };
       if constexpr (MIXED)
-        box_element_points<T>(grad, (T)(d.hx * d.hy * d.hz / 8.0), node, pt, out);
+        box_element_points(grad, (T)(d.hx * d.hy * d.hz / 8.0), node, pt, out);
       else
         box_element<T>(coef, node, pt, out);
     }
