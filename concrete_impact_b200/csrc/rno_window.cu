@@ -497,6 +497,7 @@ __device__ __forceinline__ bool run_layer_half(uint64_t* bar, uint32_t tmem, con
   return !half_sync_or(id, !ok);
 }
 
+template <bool RAW>  // raw inputs and scaled stress
 __global__ void __launch_bounds__(RW_THREADS, 1) rno_infer_kernel(const cib_rno_window w, const Scaled out, const Raw raw) {
   extern __shared__ uint8_t smem_raw[];
   InfSmem& S = *reinterpret_cast<InfSmem*>(smem_raw);
@@ -545,7 +546,7 @@ __global__ void __launch_bounds__(RW_THREADS, 1) rno_infer_kernel(const cib_rno_
 #pragma unroll
         for (int k = 0; k < 6; ++k) {
           const size_t i = (size_t)p * 6 + k;
-          if (raw.strain) {
+          if constexpr (RAW) {
             z[k] = raw.z[i];
             e[k] = normalised(raw.strain, raw.strain_f64, raw.strain_inv, raw.strain_inv32, i);
             xin[6 + k] = normalised(raw.rate, raw.rate_f64, raw.rate_inv, raw.rate_inv32, i);
@@ -558,7 +559,7 @@ __global__ void __launch_bounds__(RW_THREADS, 1) rno_infer_kernel(const cib_rno_
           xin[12 + k] = z[k];
         }
         c = w.coef[p];
-        if (raw.strain && raw.z != w.z)
+        if (RAW && raw.z != w.z)
 #pragma unroll
           for (int k = 0; k < 6; ++k) w.z[(size_t)p * 6 + k] = z[k];
       }
@@ -602,7 +603,7 @@ __global__ void __launch_bounds__(RW_THREADS, 1) rno_infer_kernel(const cib_rno_
         if (w.stress)
 #pragma unroll
           for (int k = 0; k < 6; ++k) w.stress[(size_t)p * 6 + k] = s[k];
-        if (out.stress)
+        if (RAW)
 #pragma unroll
           for (int k = 0; k < 6; ++k) out.stress[(size_t)p * 6 + k] = s[k] * out.factor;
         float* zn = w.z + (size_t)B * 6 + (size_t)p * 6;
@@ -1066,9 +1067,10 @@ int window_forward(const cib_rno_window* w, const Scaled& out, const Raw& raw, v
   if (w->T == 1 && !saves && ntiles >= 2 * (int64_t)sm_count()) {
     // inference over at least two tiles per SM: two tiles in flight per CTA
     const size_t ibytes = sizeof(InfSmem);
-    if (allow_dynamic_smem(reinterpret_cast<const void*>(rno_infer_kernel), (int)ibytes) != CIB_OK) return CIB_ECUDA;
+    auto* kernel = raw.strain ? &rno_infer_kernel<true> : &rno_infer_kernel<false>;
+    if (allow_dynamic_smem(reinterpret_cast<const void*>(kernel), (int)ibytes) != CIB_OK) return CIB_ECUDA;
     const unsigned igrid = (unsigned)std::min<int64_t>((ntiles + 1) / 2, sm_count());
-    rno_infer_kernel<<<igrid, RW_THREADS, ibytes, reinterpret_cast<cudaStream_t>(stream)>>>(*w, out, raw);
+    kernel<<<igrid, RW_THREADS, ibytes, reinterpret_cast<cudaStream_t>(stream)>>>(*w, out, raw);
     return check_launch();
   }
   if (raw.strain) {
