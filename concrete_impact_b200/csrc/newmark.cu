@@ -385,8 +385,10 @@ extern "C" int cib_csr_pcg(int64_t n, const int64_t* indptr, const int64_t* indi
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const CsrSystem a{n, indptr, indices, values, free_mask, dinv};
   const PcgGridWork w{z, r, p, work};
-  const int rc = csr_pcg_grid(a, 1, b, x, w, rtol, maxit, status, iterations, relative_residual, st);
-  if (rc != CIB_ERANGE) return rc;
+  if (b != z && b != r && b != p) {  // (the launch per phase reads b before it writes any of them)
+    const int rc = csr_pcg_grid(a, 1, b, x, w, rtol, maxit, status, iterations, relative_residual, st);
+    if (rc != CIB_ERANGE) return rc;
+  }
   return csr_pcg_launches(a, b, x, r, z, p, q, work, rtol, maxit, check_every, status, iterations, relative_residual, st);
 }
 
