@@ -288,7 +288,7 @@ def run_rve_batch(args: argparse.Namespace) -> None:
                                         "algorithmic_bytes": res_bytes},
                   "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                                "frac": None if achieved is None else achieved / peak, "traffic": None,
-                               "peak_kind": kind, "kernel": "rve_pcg_cluster_kernel<float> (rve_pcg_kernel at cluster 1)",
+                               "peak_kind": kind, "kernel": "rve_pcg_kernel<float>",
                                "algorithmic_bytes": pcg_bytes,
                                "note": "algorithmic bytes of all PCG iterations over the PCG launches' event time; "
                                        "small RVEs stay in L2"},
@@ -567,7 +567,7 @@ def run_rve_ogrid(args: argparse.Namespace) -> None:
                   "gp_evaluations_per_s": out["evaluations"] / seconds, "newton_iterations": out["newton_iterations"],
                   "final_macro_stress_pa": out["macro_stress"][-1],
                   "roofline": {"bound": "hbm", "achieved": None, "peak": None, "unit": "GB/s", "frac": None,
-                               "traffic": None, "note": "one small RVE: launch- and latency-bound CSR kernels"},
+                               "traffic": None, "note": "one small RVE: latency-bound CSR solves"},
                   "gpu_launches": out["launches"],
                   "e2e": {"value": value, "unit": "RVE steps/s", "h2d_bytes_per_step": 6 * 8,
                           "d2h_bytes_per_step": (6 + 36) * 8,
