@@ -227,12 +227,12 @@ struct Solver {
   const RvePcgArgs<T>& a;
   const RveDesc d;
   cg::cluster_group cl;
-  const int C, rank;
+  const int C, rank;  // ranks that share the system: of two or more, no one owns every layer
   int tid, warp, lane;
   int nxy, nchunk, columns, octs;  // octants of this rank
   int k0, k1;
   int prev_rank, prev_layers, next_rank;  // owners of the layers below k0 and from k1 on
-  bool wraps;     // this rank owns every layer
+  bool wraps;     // one rank owns every layer (the same on every rank: it decides barriers)
   bool lean, onchip, resident;  // resident: sp holds the slab's direction during the solve
   bool sends;     // the first node layer's direction goes to the rank below (resident, not lean)
   int kb;         // element layers per step
@@ -252,8 +252,8 @@ struct Solver {
   double* x_out;
   const double* dinv_in;
 
-  __device__ Solver(const RvePcgArgs<T>& args, const RveDesc& desc, cg::cluster_group cluster)
-      : a(args), d(desc), cl(cluster), C((int)cluster.num_blocks()), rank((int)cluster.block_rank()) {}
+  __device__ Solver(const RvePcgArgs<T>& args, const RveDesc& desc, cg::cluster_group cluster, int ranks)
+      : a(args), d(desc), cl(cluster), C(ranks), rank((int)cluster.block_rank()) {}
 
   __device__ __forceinline__ int octant_layer(int o) const { return (int)(((int64_t)o * d.nz) / OCTANTS); }
   __device__ __forceinline__ int slab_start(int q) const { return octant_layer(q * (OCTANTS / C)); }
@@ -280,14 +280,9 @@ struct Solver {
     inv_columns = 1.0f / (float)columns;
     k0 = slab_start(rank);
     k1 = slab_start(rank + 1);
-    wraps = (k1 - k0) == d.nz;
+    wraps = C == 1;
     int most = 0;
-    bool one = false;  // some rank owns every layer
-    for (int q = 0; q < C; ++q) {
-      const int layers = slab_start(q + 1) - slab_start(q);
-      most = max(most, layers);
-      one = one || layers == d.nz;
-    }
+    for (int q = 0; q < C; ++q) most = max(most, slab_start(q + 1) - slab_start(q));
     prev_rank = next_rank = rank;
     prev_layers = k1 - k0;
     if (!wraps) {  // ranks may be empty
@@ -310,7 +305,7 @@ struct Solver {
     resident = true;
     below = 0;
     int carries = 0;
-    if (!one && info_bytes(most + 1) + 2 * layer_d + (most + 2) * (layer_t + (MIXED ? layer_d : 0)) +
+    if (!wraps && info_bytes(most + 1) + 2 * layer_d + (most + 2) * (layer_t + (MIXED ? layer_d : 0)) +
                         (most + 1) * 8 * layer_t + vec_bytes <= left) {
       lean = onchip = true;
       below = 1;
@@ -322,11 +317,11 @@ struct Solver {
       const int chip = base + vec_bytes + (MIXED ? most * layer_d : 0);
       const int half = (most + 1) / 2;
       sp_layers = sp_res;
-      if (one && chip + layer_d + most * 8 * layer_t <= left) {
+      if (wraps && chip + layer_d + most * 8 * layer_t <= left) {
         onchip = true;
         carries = 1;
         kb = most;
-      } else if (one && chip + 2 * layer_d + half * 8 * layer_t <= left && half * nxy >= THREADS) {
+      } else if (wraps && chip + 2 * layer_d + half * 8 * layer_t <= left && half * nxy >= THREADS) {
         onchip = true;
         carries = 2;
         kb = half;
@@ -963,7 +958,12 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS)
     }
     return;
   }
-  Solver<T, THREADS, VEC> S(a, d, cl);
+  // A single layer has one owner: it solves alone, without a cluster barrier, and the ranks that
+  // the launcher added leave (it does not know the layers).  From two layers on two ranks or more
+  // own some, whatever C.
+  const int ranks = d.nz > 1 ? C : 1;
+  if ((int)cl.block_rank() >= ranks) return;
+  Solver<T, THREADS, VEC> S(a, d, cl, ranks);
   S.b = a.b + off;
   S.dinv = S.dinv_in = a.dinv + 3 * d.eoff;
   S.x = S.x_out = a.x + off;
@@ -982,9 +982,10 @@ int launch_shape(const RvePcgArgs<T>& a, int nsys, int max_nxy, int requested, i
   const int64_t waves = ((int64_t)nsys * cluster + sm_count() - 1) / sm_count();
   const int per_sm = waves < MIN_BLOCKS ? (int)waves : MIN_BLOCKS;
   int smem = SM_BYTES / per_sm - RESERVED - 128;
-  // one element layer, its staged direction and both carries always fit
+  // one element layer, its staged direction and both carries always fit (with the partial sums of
+  // a system that one CTA solves, where the caller asked for one)
   const int columns = max_nxy >= 32 * MAX_COLUMNS ? MAX_COLUMNS : (max_nxy + 31) / 32;
-  const int64_t least = (int64_t)PART_COUNT * (OCTANTS / cluster) * columns * 8 + (int64_t)max_nxy * (50 + 30 * sizeof(T)) + 32;
+  const int64_t least = (int64_t)PART_COUNT * (OCTANTS / requested) * columns * 8 + (int64_t)max_nxy * (50 + 30 * sizeof(T)) + 32;
   if (least > smem) smem = (int)((least + 15) & ~15LL);
   if (smem > MOST) return CIB_ERANGE;
   const int rc = allow_dynamic_smem(fn, smem > MOST ? MOST : smem);
@@ -1012,7 +1013,8 @@ int launch_shape(const RvePcgArgs<T>& a, int nsys, int max_nxy, int requested, i
 //
 // FP64: neither the shape nor the number of CTAs changes a result, so a launch that would
 // leave SMs idle gets up to 8 CTAs per system (one 8^3 system: 4.2 ms with one CTA before,
-// 0.8 ms with 8; 1 to 16 elements per CTA still gain, 4^3 0.31 ms against 0.40 with one), and
+// 0.8 ms with 8; 1 to 16 elements per CTA still gain, 4^3 0.31 ms against 0.40 with one; of a
+// system of one layer only the first CTA stays), and
 // the default block is 256 threads where an SM holds one CTA of wide layers (one 24^3 system:
 // 19.3 ms at 128 threads, 16.4 at 256) and 128 otherwise (1,152 8^3 systems: 10.0 ms against
 // 10.4; 22.8 ms with a thread per Gauss point).
