@@ -20,6 +20,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "cib_common.cuh"
 #include "umma.cuh"
 
@@ -458,6 +460,14 @@ extern "C" int cib_mlp_gemm(int32_t epilogue, int32_t M, int32_t N, int32_t K, c
   }
   const dim3 grid((unsigned)((M + 127) / 128), (unsigned)ny);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (epilogue == EPI_PARTIAL && ny < splits) {  // slices are cut at multiples of KC: the last ones may have no columns
+    const size_t first = (size_t)ny * M, row = sizeof(float) * (size_t)ldc;
+    const cudaError_t e = cudaMemset2DAsync(C + first * ldc, row, 0, std::min(row, sizeof(float) * (size_t)N), (size_t)splits * M - first, st);
+    if (e != cudaSuccess) {
+      last_cuda_error_slot() = (int)e;
+      return CIB_ECUDA;
+    }
+  }
   const int bytes = (int)sizeof(GemmSmem);
   const void* kernels[5] = {reinterpret_cast<const void*>(umma_gemm_kernel<EPI_F32>),
                             reinterpret_cast<const void*>(umma_gemm_kernel<EPI_BIAS_F32>),

@@ -434,8 +434,9 @@ int cib_rve_newton_graph_destroy(void* graph);
  *   2 Z = acc + bias (fp32; Z may be NULL), H = gelu(Z) (bf16), optional
  *     Ht[n * ldht + row_offset + m] = H
  *   3 H = acc * gelu'(Z) (bf16), optional Ht as above
- *   4 fp32 partial sums per K slice into C[(slice * M + m) * ldc + n] (splits > 1), reduced
- *     by cib_splitk_reduce in a fixed order.
+ *   4 fp32 partial sums per K slice into C[(slice * M + m) * ldc + n] for all `splits` slices
+ *     (slices are cut at multiples of 64 columns, so the last ones may have none: zeros),
+ *     reduced by cib_splitk_reduce in a fixed order.
  * err (device uint32) becomes 1 if a tensor-core completion wait exceeds 2 s (the CTA then
  * returns after releasing its tensor memory).  No reference counterpart: the reference
  * runs its surrogate through torch.nn.Linear (src/concrete_impact/nn/models/rve_rno.py:63-93). */
