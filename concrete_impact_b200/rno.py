@@ -25,7 +25,7 @@ import numpy as np
 import torch
 
 from . import _native
-from .mlp import EPI_BIAS_F32, EPI_BIAS_GELU, EPI_F32, EPI_GELU_BWD, EPI_PARTIAL, gemm, splitk_reduce
+from .mlp import EPI_BIAS_F32, EPI_BIAS_GELU, EPI_F32, EPI_GELU_BWD, gemm
 
 IN_REAL, IN_PAD, OUT_REAL, OUT_PAD = 18, 32, 12, 16
 
@@ -202,8 +202,6 @@ class RNOSurrogate:
             return torch.zeros(shape, dtype=dtype, device=dev)
 
         splits = max(1, min(64, Rp // 512))
-        per = -(-(-(-Rp // splits)) // 64) * 64  # K columns per slice, as the kernels cut them
-        fused_slices = -(-Rp // per) == splits
         self._window = {
             "T": T, "B": B, "R": R, "Rp": Rp, "splits": splits,
             "strain": e(T, B, 6), "rate": e(T, B, 6), "target": e(T, B, 6), "coef": e(T, B), "z": e(T + 1, B, 6),
@@ -215,8 +213,8 @@ class RNOSurrogate:
             "dY": e(B, OUT_PAD, dtype=bf), "dYt": e(OUT_PAD, Rp, dtype=bf),
             "dZ": [e(B, h, dtype=bf) for _ in range(3)], "dZt": [e(h, Rp, dtype=bf) for _ in range(3)],
             "dX": e(B, IN_PAD), "dz": [e(B, 6), e(B, 6)],
-            "partial": e(splits * (sum(L.w.numel() for L in self.layers) if fused_slices else h * h)),
-            "row_partial": torch.zeros(splits * 512, dtype=torch.float64, device=dev), "fused_slices": fused_slices,
+            "partial": e(splits * sum(L.w.numel() for L in self.layers)),
+            "row_partial": torch.zeros(splits * 512, dtype=torch.float64, device=dev),
         }  # fmt: skip
         self._graph = None
         return self._window
@@ -309,34 +307,21 @@ class RNOSurrogate:
             dz_next, dz = dz, dz_next
 
     def _weight_gradients(self, w: dict) -> None:
-        """Weight and bias gradients over all rows of the window (split-K products).  Windows
-        whose rows fill every K slice take all layers in one launch and one reduction (512 paths
-        x 50 steps: 183 us in twelve launches, 42 in two).  The others keep the product per
-        layer: its reduction also reads the slices beyond the last one written, so its last
-        layer's sums are not those of the fused form."""
-        lib = self.lib
-        sp = _native.stream_ptr()
+        """Weight and bias gradients over all rows of the window: the split-K products of all
+        layers in one launch, their sums over the slices in another (512 paths x 50 steps: 183 us
+        in a launch per product, reduction and row sum, 42 us in two)."""
         ins = [w["Xt"], w["Ht"][0], w["Ht"][1], w["Ht"][2]]
         outs = [w["dZt"][0], w["dZt"][1], w["dZt"][2], w["dYt"]]
-        if w["fused_slices"]:
-            c = _native.RNOWgradC()
-            c.K = c.ld = w["Rp"]
-            c.splits = w["splits"]
-            for i, L in enumerate(self.layers):
-                c.M[i], c.N[i] = L.w.shape
-                c.A[i], c.B[i] = outs[i].data_ptr(), ins[i].data_ptr()
-                c.gw[i], c.gb[i] = L.gw.data_ptr(), L.gb.data_ptr()
-            c.partial, c.row_partial = w["partial"].data_ptr(), w["row_partial"].data_ptr()
-            c.err = self.err.data_ptr()
-            _check(lib.cib_rno_weight_gradients(ctypes.byref(c), sp), "cib_rno_weight_gradients")
-            return
-        h = self.config.hidden
+        c = _native.RNOWgradC()
+        c.K = c.ld = w["Rp"]
+        c.splits = w["splits"]
         for i, L in enumerate(self.layers):
-            m, n = L.w.shape
-            part = w["partial"].view(-1, h)[: w["splits"] * m]
-            gemm(EPI_PARTIAL, outs[i], ins[i], c=part, splits=w["splits"], err=self.err, rows=m)
-            splitk_reduce(part.view(w["splits"], m, n) if n == h else part, w["splits"], m, n, L.gw)
-            _check(lib.cib_row_sum_bf16(m, w["R"], outs[i].data_ptr(), w["Rp"], L.gb.data_ptr(), sp), "cib_row_sum_bf16")
+            c.M[i], c.N[i] = L.w.shape
+            c.A[i], c.B[i] = outs[i].data_ptr(), ins[i].data_ptr()
+            c.gw[i], c.gb[i] = L.gw.data_ptr(), L.gb.data_ptr()
+        c.partial, c.row_partial = w["partial"].data_ptr(), w["row_partial"].data_ptr()
+        c.err = self.err.data_ptr()
+        _check(self.lib.cib_rno_weight_gradients(ctypes.byref(c), _native.stream_ptr()), "cib_rno_weight_gradients")
 
     def _adam(self) -> None:
         lib, sp, c = self.lib, _native.stream_ptr(), self.config
