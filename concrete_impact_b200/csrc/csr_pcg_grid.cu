@@ -123,7 +123,7 @@ __device__ __forceinline__ bool get(const Word* lo, const Word* hi, const int64_
         v[k] = __longlong_as_double((long long)((h[k] << 32) | (l[k] & 0xffffffffull)));
         waiting &= ~(1u << k);
       }
-    if ((++tries & 1023) == 0) {
+    if (waiting && (++tries & 1023) == 0) {
       const unsigned long long now = now_ns();
       if (since == 0) since = now;
       if (now - since > WAIT_NS) return false;

@@ -371,6 +371,32 @@ int csr_pcg_launches(const CsrSystem& a, const double* b, double* x, double* r, 
   return CIB_OK;
 }
 
+// One right-hand side.  `persistent`: whether to offer the system to the persistent solve, and
+// whether that took it.  It gives a system back when some CTA's rows do not fit, after the other
+// CTAs have written their part of the solution: where b is x, that goes to q (which it does not
+// use) and from there to x.  b may also be r, z or p: those it overwrites first, and the launch
+// per phase reads b before it writes them.
+int csr_pcg_one(const CsrSystem& a, const double* b, double* x, double* r, double* z, double* p, double* q, double* work,
+                double rtol, int32_t maxit, int32_t check_every, int32_t* status, int32_t* iterations,
+                double* relative_residual, cudaStream_t st, bool& persistent) {
+  persistent = persistent && b != z && b != r && b != p;
+  if (persistent) {
+    const PcgGridWork w{z, r, p, work};
+    double* out = b == x ? q : x;
+    const int rc = csr_pcg_grid(a, 1, b, out, w, rtol, maxit, status, iterations, relative_residual, st);
+    if (rc == CIB_OK && out != x) {
+      const cudaError_t e = cudaMemcpyAsync(x, out, sizeof(double) * (size_t)a.n, cudaMemcpyDeviceToDevice, st);
+      if (e != cudaSuccess) {
+        last_cuda_error_slot() = (int)e;
+        return CIB_ECUDA;
+      }
+    }
+    if (rc != CIB_ERANGE) return rc;
+    persistent = false;
+  }
+  return csr_pcg_launches(a, b, x, r, z, p, q, work, rtol, maxit, check_every, status, iterations, relative_residual, st);
+}
+
 }  // namespace
 }  // namespace cib
 
@@ -382,14 +408,10 @@ extern "C" int cib_csr_pcg(int64_t n, const int64_t* indptr, const int64_t* indi
   if (n <= 0 || !indptr || !indices || !values || !free_mask || !dinv || !b || !x || !r || !z || !p || !q || !work ||
       !status || !iterations || !relative_residual || maxit < 0 || check_every <= 0 || !(rtol >= 0.0))
     return CIB_EINVAL;
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const CsrSystem a{n, indptr, indices, values, free_mask, dinv};
-  const PcgGridWork w{z, r, p, work};
-  if (b != z && b != r && b != p) {  // (the launch per phase reads b before it writes any of them)
-    const int rc = csr_pcg_grid(a, 1, b, x, w, rtol, maxit, status, iterations, relative_residual, st);
-    if (rc != CIB_ERANGE) return rc;
-  }
-  return csr_pcg_launches(a, b, x, r, z, p, q, work, rtol, maxit, check_every, status, iterations, relative_residual, st);
+  bool persistent = true;
+  return csr_pcg_one(a, b, x, r, z, p, q, work, rtol, maxit, check_every, status, iterations, relative_residual,
+                     reinterpret_cast<cudaStream_t>(stream), persistent);
 }
 
 extern "C" int cib_csr_pcg_block(int64_t n, const int64_t* indptr, const int64_t* indices, const double* values,
@@ -402,14 +424,19 @@ extern "C" int cib_csr_pcg_block(int64_t n, const int64_t* indptr, const int64_t
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const CsrSystem a{n, indptr, indices, values, free_mask, dinv};
   double* vectors = work + CIB_CSR_PCG_BLOCK_WORK_DOUBLES(0);  // 12 n
-  const PcgGridWork w{vectors, vectors + PCG_BLOCK_RHS * n, work, work + BLOCK_PART};
-  int rc = csr_pcg_grid(a, PCG_BLOCK_RHS, b, x, w, rtol, maxit, status, iterations, relative_residual, st);
-  for (int j = 0; rc == CIB_ERANGE && j < PCG_BLOCK_RHS; ++j) {
-    rc = cib_csr_pcg(n, indptr, indices, values, free_mask, dinv, b + j * n, x + j * n, vectors, vectors + n,
-                     vectors + 2 * n, vectors + 3 * n, work, rtol, maxit, check_every, status + j, iterations + j,
-                     relative_residual + j, stream);
-    if (rc != CIB_OK) return rc;
-    rc = CIB_ERANGE;
+  if (b != x) {  // (a solve that is given back may have written to x)
+    const PcgGridWork w{vectors, vectors + PCG_BLOCK_RHS * n, work, work + BLOCK_PART};
+    const int rc = csr_pcg_grid(a, PCG_BLOCK_RHS, b, x, w, rtol, maxit, status, iterations, relative_residual, st);
+    if (rc != CIB_ERANGE) return rc;
   }
-  return rc == CIB_ERANGE ? CIB_OK : rc;
+  // One by one; the persistent solve of one keeps less per column and may take what that of six
+  // does not.  What it gives back once it would give back six times (20,000 rows of 81 scattered
+  // columns: 37 us each).
+  bool persistent = true;
+  for (int j = 0; j < PCG_BLOCK_RHS; ++j) {
+    const int rc = csr_pcg_one(a, b + j * n, x + j * n, vectors, vectors + n, vectors + 2 * n, vectors + 3 * n, work, rtol,
+                               maxit, check_every, status + j, iterations + j, relative_residual + j, st, persistent);
+    if (rc != CIB_OK) return rc;
+  }
+  return CIB_OK;
 }

@@ -607,7 +607,8 @@ int cib_csr_spmv(int64_t n, const int64_t* indptr, const int64_t* indices, const
  * check_every iterations.  Host outputs: status 0 converged, 1 iteration limit, 2 breakdown
  * (p.Ap <= 0 or a non-finite value); iterations; relative_residual ||r|| / ||b||.  Up to
  * 28,416 rows the solve is one cooperative launch, read once at its end (check_every then has
- * no effect).  The dot products are reduced in a fixed order: bitwise repeatable.  Returns CIB_ERANGE when n
+ * no effect).  The dot products are reduced in a fixed order: bitwise repeatable.  b may be x or
+ * one of r, z, p, q (the same address); no other two arrays overlap.  Returns CIB_ERANGE when n
  * needs more than CIB_CSR_PCG_MAX_GRID blocks of partials. */
 #define CIB_CSR_PCG_MAX_GRID 1024
 #define CIB_CSR_PCG_WORK_DOUBLES (3 * CIB_CSR_PCG_MAX_GRID + 8)
@@ -631,7 +632,8 @@ int cib_copy_rows(int64_t count, const int64_t* ids, int32_t arrays, const cib_r
 
 /* Six right-hand sides of one matrix (rows of b and x, 6 x n): as six calls of cib_csr_pcg, in
  * one pass over the matrix where that takes the system.  status, iterations and
- * relative_residual hold six entries; work CIB_CSR_PCG_BLOCK_WORK_DOUBLES(n) doubles. */
+ * relative_residual hold six entries; work CIB_CSR_PCG_BLOCK_WORK_DOUBLES(n) doubles.  b may be x
+ * (the six are then solved one by one); no other two arrays overlap. */
 #define CIB_CSR_PCG_BLOCK_WORK_DOUBLES(n) (12 * (n) + 24576)
 int cib_csr_pcg_block(int64_t n, const int64_t* indptr, const int64_t* indices, const double* values,
                       const uint8_t* free_mask, const double* dinv, const double* b, double* x, double* work,
