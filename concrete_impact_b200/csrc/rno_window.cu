@@ -1107,6 +1107,9 @@ extern "C" int cib_rno_window_forward(const cib_rno_window* w, void* stream) {
 extern "C" int cib_rno_predict(const cib_rno_window* w, const cib_rno_predict_inputs* in, void* stream) {
   if (validate_common(w) != CIB_OK || w->T != 1 || !in || !in->strain || !in->rate || !in->z || !in->stress)
     return CIB_EINVAL;
+  // w.z[0] and w.z[1] are written point by point: a state that is not one of them lies outside
+  const float *first = w->z, *second = first + 6 * (int64_t)w->B, *end = second + 6 * (int64_t)w->B;
+  if (in->z != first && in->z != second && in->z < end && in->z + 6 * (int64_t)w->B > first) return CIB_EINVAL;
   if (w->B == 0) return CIB_OK;
   Raw raw;
   raw.strain = in->strain, raw.rate = in->rate, raw.z = in->z;

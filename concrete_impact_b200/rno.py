@@ -514,7 +514,7 @@ class RNOSurrogate:
         c.skip = None if self.skip is None else self.skip.data_ptr()
         c.stress = buffers["stress"].data_ptr()
         c.err = self.err.data_ptr()
-        if self._raw_inputs(strain, rate, z, M):
+        if self._raw_inputs(strain, rate, z, buffers["z"]):
             scratch = torch.empty((2, M, 6), dtype=torch.float32, device=dev)
             out = torch.empty((M, 6), dtype=torch.float32, device=dev)
             c.strain, c.rate = scratch[0].data_ptr(), scratch[1].data_ptr()
@@ -529,12 +529,20 @@ class RNOSurrogate:
         _check(self.lib.cib_rno_window_forward(ctypes.byref(c), _native.stream_ptr()), "cib_rno_window_forward")
         return buffers["stress"][0] * s.stress, buffers["z"][1], buffers
 
-    def _raw_inputs(self, strain: torch.Tensor, rate: torch.Tensor, z: torch.Tensor, M: int) -> bool:
-        """Whether the step can take its inputs as they are: contiguous (M, 6) on the device,
-        strain and rate FP32 or FP64, the latent state FP32.  Anything else goes through torch."""
-        kinds = ((strain, (torch.float32, torch.float64)), (rate, (torch.float32, torch.float64)), (z, (torch.float32,)))
-        return M > 0 and all(t.shape == (M, 6) and t.is_cuda and t.is_contiguous() and t.dtype in kind and not t.requires_grad
-                             for t, kind in kinds)  # fmt: skip
+    def _raw_inputs(self, strain: torch.Tensor, rate: torch.Tensor, z: torch.Tensor, states: torch.Tensor) -> bool:
+        """Whether the step can take its inputs as they are: contiguous (M, 6) on the buffers'
+        device, strain and rate FP32 or FP64, the latent state FP32, all of them outside the two
+        ``states`` (2, M, 6) that the step writes point by point (the latent state may be one of
+        the two).  Anything else goes through torch."""
+        wide, begin, size = (torch.float32, torch.float64), states.data_ptr(), states.numel() * 4
+        for t, kinds in ((strain, wide), (rate, wide), (z, wide[:1])):
+            if not (t.shape == states.shape[1:] and t.device == states.device and t.is_contiguous() and t.dtype in kinds
+                    and not t.requires_grad):  # fmt: skip
+                return False
+            at = t.data_ptr() - begin
+            if -t.numel() * t.element_size() < at < size and not (t is z and at in (0, size // 2)):
+                return False
+        return size > 0
 
     def predict_normalized(self, strain_n: torch.Tensor, rate_n: torch.Tensor, coef: torch.Tensor, z: torch.Tensor,
                            stress_n: torch.Tensor) -> None:  # fmt: skip

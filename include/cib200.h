@@ -521,8 +521,8 @@ int cib_rno_window_forward(const cib_rno_window* w, void* stream);
 
 /* One step (w->T = 1) from physical inputs: strain and rate (B, 6), each FP64 or FP32, are
  * divided by their scales into the buffers w->strain and w->rate, the latent state z (B, 6) is
- * copied to w->z[0] (z may be any part of w->z), and stress (B, 6) receives the stress times
- * stress_scale. */
+ * copied to w->z[0], and stress (B, 6) receives the stress times stress_scale.  z may be w->z[0]
+ * or w->z[1]; another part of w->z is CIB_EINVAL, and no other input overlaps an output. */
 typedef struct cib_rno_predict_inputs {
   const void* strain;
   const void* rate;
