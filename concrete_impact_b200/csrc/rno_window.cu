@@ -870,7 +870,7 @@ __global__ void __launch_bounds__(NW_THREADS, 1) rno_narrow_forward_kernel(const
       }
       __syncthreads();  // S.y
     }
-    // window loss of this tile: row tile % 8 of loss_part, whose remaining rows are zero
+    // window loss of this tile: row tile % 8 of loss_part; narrow_loss_kernel adds the rows
     if (w.loss_part && run) {
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
@@ -879,11 +879,8 @@ __global__ void __launch_bounds__(NW_THREADS, 1) rno_narrow_forward_kernel(const
       if (tid == 0) {
         double tot = 0.0;
         for (int i = 0; i < NW_THREADS / 32; ++i) tot += S.red[i];
-        const int wide = (B + TILE - 1) / TILE, col = tile / (TILE / NP), row = tile % (TILE / NP);
-        w.loss_part[(size_t)row * wide + col] = tot;
-        if (row == 0)
-          for (int r = 1; r < T; ++r)
-            if (r >= TILE / NP || col * (TILE / NP) + r >= ntiles) w.loss_part[(size_t)r * wide + col] = 0.0;
+        const int wide = (B + TILE - 1) / TILE;
+        w.loss_part[(size_t)(tile % (TILE / NP)) * wide + tile / (TILE / NP)] = tot;
       }
     }
     __syncthreads();  // the last step's S.y and S.red are read
@@ -895,6 +892,21 @@ __global__ void __launch_bounds__(NW_THREADS, 1) rno_narrow_forward_kernel(const
     fence_after_sync();
     tmem_dealloc(tmem, 32);
   }
+}
+
+// Row 0 of loss_part becomes the loss of each group of 128 paths, the sum of its tiles of 16 in
+// order; the other rows zero.
+__global__ void __launch_bounds__(128) narrow_loss_kernel(int B, int T, double* __restrict__ loss_part) {
+  const int wide = (B + TILE - 1) / TILE, col = blockIdx.x * blockDim.x + threadIdx.x;
+  if (col >= wide) return;
+  const int tiles = min(TILE / NP, (B - col * TILE + NP - 1) / NP);
+  double v[TILE / NP], sum = 0.0;
+#pragma unroll
+  for (int r = 0; r < TILE / NP; ++r) v[r] = r < tiles ? loss_part[(size_t)r * wide + col] : 0.0;
+#pragma unroll
+  for (int r = 0; r < TILE / NP; ++r) sum += v[r];
+  loss_part[col] = sum;
+  for (int r = 1; r < T; ++r) loss_part[(size_t)r * wide + col] = 0.0;
 }
 
 // The thread of column 6 + k of the output-gradient tile keeps dz_k of its path.
@@ -1079,13 +1091,16 @@ int window_forward(const cib_rno_window* w, const Scaled& out, const Raw& raw, v
         n, raw, const_cast<float*>(w->strain), const_cast<float*>(w->rate), w->z);
     if (check_launch() != CIB_OK) return CIB_ECUDA;
   }
-  // (its loss grouping needs 8 rows of loss_part)
+  // (the losses of its tiles need 8 rows of loss_part)
   if (narrow_window(w->B) && (!w->loss_part || w->T >= TILE / NP)) {
     const size_t nbytes = sizeof(NarrowFwdSmem);
     if (allow_dynamic_smem(reinterpret_cast<const void*>(rno_narrow_forward_kernel), (int)nbytes) != CIB_OK)
       return CIB_ECUDA;
     const unsigned ngrid = (unsigned)std::min<int64_t>((w->B + NP - 1) / NP, sm_count());
     rno_narrow_forward_kernel<<<ngrid, NW_THREADS, nbytes, reinterpret_cast<cudaStream_t>(stream)>>>(*w, out);
+    const int rc = check_launch();
+    if (rc != CIB_OK || !w->loss_part) return rc;
+    narrow_loss_kernel<<<(unsigned)((ntiles + 127) / 128), 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(w->B, w->T, w->loss_part);
     return check_launch();
   }
   const size_t bytes = sizeof(FwdSmem);

@@ -487,8 +487,8 @@ int cib_counter_increment(int32_t* counter, void* stream);
  * pre-activations; Xt (32, ldt), Ht[l] (128, ldt), dYt (16, ldt), dZt[l] (128, ldt) bf16
  * transposes with column t B + p.  Optional outputs may be NULL in the forward (Z, Xt, Ht,
  * stress, target/gS/loss_part); the backward needs Wt, Z, gS, dYt and dZt.
- * loss_part (T, ceil(B / 128)): row 0 holds each CTA's sum of squared errors over the
- * window, the other rows zero.  gS = loss_scale * 2 (s - target).  The backward runs the
+ * loss_part (T, ceil(B / 128)): row 0 holds each group of 128 paths' sum of squared errors over
+ * the window, the other rows zero.  gS = loss_scale * 2 (s - target).  The backward runs the
  * window in reverse with dz(T) = 0 and writes dY^T, dZ^T for the weight-gradient GEMMs.
  * err (device uint32) becomes 1 when a tensor-core wait exceeds 2 s.  No reference
  * counterpart (the reference runs torch.nn layers per step). */
