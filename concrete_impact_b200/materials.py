@@ -25,6 +25,7 @@ from typing import Any, NamedTuple, Protocol
 
 import numpy as np
 import torch
+import torch.autograd.forward_ad as fwd
 
 from . import _native
 
@@ -516,6 +517,12 @@ class RVEPhase:
     material: MaterialModel
 
 
+def _transforming() -> bool:
+    """Whether forward mode or a torch.func transform is active.  Then, and where a tensor requires
+    a gradient, values go through torch's own operations."""
+    return fwd._current_level >= 0 or torch._C._are_functorch_transforms_active()
+
+
 class _Everywhere(NamedTuple):
     """A diagnostic with one value at all points of a phase."""
 
@@ -569,7 +576,9 @@ class PhasedMaterialModel:
         ids_of = [np.flatnonzero(phase_ids == phase_id) for phase_id in range(len(self.phases))]
         new = torch.empty if sum(ids.size for ids in ids_of) == point_count else torch.zeros  # points of no phase: zeros
         where = dict(dtype=torch.float64, device=io.device)
-        stresses = new(eps.shape, **where)
+        transforming = _transforming()
+        tracked = transforming or eps.requires_grad or (rates is not None and rates.requires_grad)
+        stresses = torch.zeros_like(eps) if tracked else new(eps.shape, **where)
         tangents = new((point_count, component_count, component_count), **where) if requirements.tangent else None
         free_energy = new(point_count, **where) if requirements.free_energy else None
         dissipation = new(point_count, **where) if requirements.dissipation else None
@@ -578,9 +587,12 @@ class PhasedMaterialModel:
         for phase, phase_points in zip(self.phases, ids_of):
             ids = torch.as_tensor(phase_points, device=io.device)
             phase_state = _decode_phase_state(state, phase.name)
-            inputs = [None if a is None else io.empty(ids.numel(), component_count) for a in (eps, rates)]
-            _native.copy_rows(ids, [(a, to, component_count, 0.0) for a, to in zip((eps, rates), inputs) if a is not None],
-                              scatter=False)  # fmt: skip
+            if tracked:
+                inputs = [None if a is None else a.index_select(0, ids) for a in (eps, rates)]
+            else:
+                inputs = [None if a is None else io.empty(ids.numel(), component_count) for a in (eps, rates)]
+                _native.copy_rows(ids, [(a, to, component_count, 0.0) for a, to in zip((eps, rates), inputs) if a is not None],
+                                  scatter=False)  # fmt: skip
             phase_request = MaterialPointRequest(
                 strains=inputs[0],
                 strain_rates=inputs[1],
@@ -612,11 +624,16 @@ class PhasedMaterialModel:
                     fields.append((to, value))
             for name, values in response.state.variables.items():
                 next_variables[encode_phase_state_key(phase.name, name)] = io.out(values)
-            results.append((ids, fields, diagnostics))
+            results.append((ids, fields, {name: values if isinstance(values, _Everywhere) else io.to_device(values)
+                                          for name, values in diagnostics.items()}))  # fmt: skip
         names = sorted(set().union(*(d.keys() for _, _, d in results)))
         missing = _Everywhere(float("nan"))
         block = torch.full((len(names), point_count), missing.value, **where) if new is torch.zeros else io.empty(len(names), point_count)
         combined = dict(zip(names, block))
+        for _, _, diagnostics in results:
+            for name, values in diagnostics.items():
+                if not isinstance(values, _Everywhere) and (transforming or values.requires_grad):
+                    combined[name] = torch.full((point_count,), missing.value, **where)  # not a view of the others' block
         for ids, fields, diagnostics in results:
             copies = []
             for name, to in combined.items():
@@ -624,9 +641,10 @@ class PhasedMaterialModel:
                 if isinstance(values, _Everywhere):
                     copies.append((None, to, 1, values.value))
                 else:
-                    fields.append((to, io.to_device(values)))
+                    fields.append((to, values))
             for to, values in fields:
-                if values.shape == (ids.numel(), *to.shape[1:]) and values.dtype == torch.float64 and values.is_cuda:
+                if (values.shape == (ids.numel(), *to.shape[1:]) and values.dtype == torch.float64
+                        and values.device == to.device and not (transforming or values.requires_grad)):  # fmt: skip
                     copies.append((values.contiguous(), to, math.prod(to.shape[1:]), 0.0))
                 else:
                     to.index_copy_(0, ids, values)
