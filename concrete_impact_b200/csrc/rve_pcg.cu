@@ -1018,7 +1018,8 @@ int launch_shape(const RvePcgArgs<T>& a, int nsys, int max_nxy, int requested, i
 // the default block is 256 threads where an SM holds one CTA of wide layers (one 24^3 system:
 // 19.3 ms at 128 threads, 16.4 at 256) and 128 otherwise (1,152 8^3 systems: 10.0 ms against
 // 10.4; 22.8 ms with a thread per Gauss point).
-// FP32: dot products are summed per block and rank, so both are taken as given.
+// FP32: dot products are summed per block and rank, so both are taken as given; the shape applies
+// to two CTAs or more (one CTA is the solve of cib_rve_pcg).
 template <typename T>
 int launch_rve_pcg_cluster(const RvePcgArgs<T>& a, int nsys, int max_nxy, int cluster, cudaStream_t st) {
   const int c = cluster & 15, shape = (cluster >> 4) & 15;
@@ -1029,7 +1030,7 @@ int launch_rve_pcg_cluster(const RvePcgArgs<T>& a, int nsys, int max_nxy, int cl
   if ((size_t)max_nxy * layer > 200 * 1024) return CIB_ERANGE;
   const bool vec = aligned16(a.tparam) && (a.ngp % (16 / (int)sizeof(T))) == 0;  // rows of 16-byte loads
   if constexpr (sizeof(T) == 4) {
-    switch (shape) {
+    switch (c == 1 ? 0 : shape) {
       case 1:
         return vec ? launch_shape<T, 128, 4, true>(a, nsys, max_nxy, c, c, st)
                    : launch_shape<T, 128, 4, false>(a, nsys, max_nxy, c, c, st);

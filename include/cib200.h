@@ -315,8 +315,8 @@ int cib_rve_pcg(const cib_rve_batch* batch, int32_t nsys, const int32_t* sys_rve
 /* cib_rve_pcg with `cluster` (1, 2, 4 or 8) CTAs of one thread-block cluster per system:
  * each CTA owns a slab of z node layers, slab boundaries are exchanged and the dot
  * products combined through distributed shared memory in a fixed order.  Every RVE needs
- * nz >= cluster (else that system's status is 3); cluster 1 is cib_rve_pcg.  Bits 4-7 of
- * `cluster` select the threads per CTA: 0 the default (256 in FP32; 128 or 256 by the grid in
+ * nz >= cluster (else that system's status is 3); cluster 1 is cib_rve_pcg, whatever the shape.
+ * Bits 4-7 of `cluster` select the threads per CTA: 0 the default (256 in FP32; 128 or 256 by the grid in
  * FP64), 1 128, 2 512 in FP32 and 256 in FP64, 3 256 in FP32 and 64 in FP64.  FP64 results are
  * bitwise the same for every cluster size and shape (a grid that would leave SMs idle gets up
  * to 8 CTAs per system whatever `cluster` asks for); FP32 results are reproducible for given
