@@ -34,6 +34,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <type_traits>
 
 #include "cib_common.cuh"
@@ -1006,13 +1007,45 @@ int launch_shape(const RvePcgArgs<T>& a, int nsys, int max_nxy, int requested, i
   return check_launch();
 }
 
+// Clusters of C CTAs, an SM's whole shared memory each, that run at the same time: fewer than
+// sm_count() / C, as a cluster stays within a GPC (15 of 8 and 33 of 4 on the B200s measured).
+// Beyond them a launch takes a second turn: 18 systems of 8^3 in clusters of 8 1.54 ms, of 4
+// 0.98; 36 in clusters of 4 1.83 ms, of 2 1.33.  Kept per device; 0 where none runs.
+int resident_clusters(int C) {
+  static std::atomic<int> kept[64][9];  // 1 + the number
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  if (const int k = kept[dev][C].load()) return k - 1;
+  const auto fn = rve_pcg_kernel<double, 128, 2, true>;
+  constexpr int SMEM = 227 * 1024;
+  if (allow_dynamic_smem(reinterpret_cast<const void*>(fn), SMEM) != CIB_OK) return 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)C, 1, 1);
+  cfg.blockDim = dim3(128, 1, 1);
+  cfg.dynamicSmemBytes = SMEM;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)C;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    n = 0;
+  }
+  kept[dev][C].store(1 + n);
+  return n;
+}
+
 }  // namespace
 
 // cluster: the CTAs per system (1, 2, 4 or 8) in bits 0-3 and the launch shape in bits 4-7
 // (block size: 0 the default, 1 128 threads, 2 FP32 512 / FP64 256, 3 FP32 256 / FP64 64).
 //
 // FP64: neither the shape nor the number of CTAs changes a result, so a launch that would
-// leave SMs idle gets up to 8 CTAs per system (one 8^3 system: 4.2 ms with one CTA before,
+// leave SMs idle gets up to 8 CTAs per system while all clusters run at once (one 8^3 system: 4.2 ms with one CTA before,
 // 0.8 ms with 8; 1 to 16 elements per CTA still gain, 4^3 0.31 ms against 0.40 with one; of a
 // system of one layer only the first CTA stays), and
 // the default block is 256 threads where an SM holds one CTA of wide layers (one 24^3 system:
@@ -1043,7 +1076,7 @@ int launch_rve_pcg_cluster(const RvePcgArgs<T>& a, int nsys, int max_nxy, int cl
     }
   } else {
     int C = c;
-    while (C < 8 && (int64_t)nsys * (2 * C) <= sm_count()) C *= 2;
+    while (C < 8 && (int64_t)nsys * (2 * C) <= sm_count() && nsys <= resident_clusters(2 * C)) C *= 2;
     if (!vec) return launch_shape<T, 128, 2, false>(a, nsys, max_nxy, c, C, st);
     const bool wide = (int64_t)nsys * C <= sm_count() && max_nxy >= 256;
     if (shape == 3) return launch_shape<T, 64, 4, true>(a, nsys, max_nxy, c, C, st);
