@@ -216,8 +216,9 @@ __device__ __forceinline__ bool opaque(bool v) {
 // memory (the rule is in plan()):
 //  * lean: several ranks, every vector of the slab on chip.  The rank also applies the element
 //    layer below its slab and keeps the direction of the node layers on both sides, which it
-//    updates itself from the z = dinv r that its neighbours send with their r update: an
-//    iteration then needs only the two cluster barriers of its dot products.
+//    updates itself, as their owners do, from the z = dinv r (FP32: the r) that its neighbours
+//    send with their r update: an iteration then needs only the two cluster barriers of its dot
+//    products.
 //  * on chip: the same vectors in shared memory on a single rank, in one or two steps.
 //  * otherwise the vectors stay in global memory (L2); ranks exchange the contributions to
 //    their first node layer and the direction above their last through shared memory.
@@ -235,6 +236,7 @@ struct Solver {
   int prev_rank, prev_layers, next_rank;  // owners of the layers below k0 and from k1 on
   bool wraps;     // one rank owns every layer (the same on every rank: it decides barriers)
   bool lean, onchip, resident;  // resident: sp holds the slab's direction during the solve
+  bool wide;      // MIXED, lean: dinv of the layers beside the slab is on chip as well
   bool sends;     // the first node layer's direction goes to the rank below (resident, not lean)
   int kb;         // element layers per step
   int below;      // 1 when sp, ye and info begin at layer k0 - 1 (lean), else 0
@@ -243,7 +245,8 @@ struct Solver {
   // shared memory
   double* parts;   // [PART_COUNT][octs * columns]
   double* carry;   // [1 or 2][3 nxy]: contributions of a step's last element layer to the next node layer
-  double* halo;    // lean: z of node layers k0 - 1 and k1, [2][3 nxy], written by the neighbours
+  double* halo;    // lean: z of node layers k0 - 1 and k1, [2][3 nxy], written by the neighbours (MIXED: r
+                   // has these layers, and dinv where `wide`)
   T* sp;           // [sp_layers][3 nxy] search direction
   T* ye;           // [24][es] element contributions
   uint16_t* info;  // flags of the 8 points | phase << 8 per element of the slab (not resident: of the step)
@@ -306,8 +309,11 @@ struct Solver {
     resident = true;
     below = 0;
     int carries = 0;
-    if (!wraps && info_bytes(most + 1) + 2 * layer_d + (most + 2) * (layer_t + (MIXED ? layer_d : 0)) +
-                        (most + 1) * 8 * layer_t + vec_bytes <= left) {
+    const int lean_bytes = info_bytes(most + 1) + 2 * layer_d + (most + 2) * (layer_t + (MIXED ? layer_d : 0)) +
+                           (most + 1) * 8 * layer_t + vec_bytes;
+    wide = false;
+    if (!wraps && lean_bytes <= left) {
+      wide = MIXED && lean_bytes + 2 * layer_d <= left;
       lean = onchip = true;
       below = 1;
       kb = most + 1;
@@ -355,12 +361,12 @@ struct Solver {
     const int64_t row = 3 * (int64_t)nxy, own = row * k0;
     parts = take(part_count);
     carry = take(carries * row);
-    halo = lean ? take(2 * row) : nullptr;
+    if (!MIXED) halo = lean ? take(2 * row) : nullptr;
     if (onchip) {
-      r = take(most * row) - own;
+      r = take((most + (MIXED ? 2 * below : 0)) * row) + (MIXED ? below : 0) * row - own;
       Ap = take(most * row) - own;
       x = take(most * row) - own;
-      dinv = take(most * row) - own;
+      dinv = take((most + 2 * wide) * row) + wide * row - own;
       if (MIXED) p = take((most + 2 * below) * row) + below * row - own;
     }
     sp = reinterpret_cast<T*>(at);
@@ -644,24 +650,34 @@ struct Solver {
     }
   }
 
-  // Lean: the direction of the node layers beside the slab, z + beta p (z from global memory
-  // on the first call).
-  __device__ __forceinline__ void halo_direction(double beta, bool first) {
-    const int row = 3 * nxy;
+  // The next direction, dinv r + beta p.  Its owner and, beside a slab, a neighbour form it, and
+  // the launch decides where that is: the operations are named, so that every launch rounds
+  // alike.  FP32 Newton steps stop on thresholds and keep the form that rounds the owner's
+  // product last (4e-6 of a batch's results hang on it); FP64 needs z only.
+  __device__ __forceinline__ static double next_direction(double di, double r, double beta, double p) {
+    return MIXED ? fma(di, r, __dmul_rn(beta, p)) : fma(beta, p, __dmul_rn(di, r));
+  }
+
+  // Lean: the direction of the node layers beside the slab, half of the threads each.
+  __device__ __forceinline__ void halo_direction(double beta) {
+    const int row = 3 * nxy, side = tid >= THREADS / 2;
+    const int k = side ? k1 : k0 - 1;
+    T* to = sp + (side ? k1 - k0 + 1 : 0) * row;
+    if constexpr (MIXED) {
+      const int64_t i = (int64_t)row * k;
+      const double* di = wide ? dinv + i : dinv_in + (int64_t)row * wrap_layer(k);
+      const double* ri = r + i;
+      double* pi = p + i;
 #pragma unroll 1
-    for (int t = tid; t < 2 * row; t += THREADS) {
-      const int side = t >= row, f = t - side * row;
-      const int k = side ? k1 : k0 - 1, l = side ? k1 - k0 + 1 : 0;
-      double v;
-      if (opaque(first)) {
-        const int64_t g = (int64_t)row * wrap_layer(k) + f;
-        v = dinv_in[g] * b[g];
-      } else {
-        const double old = MIXED ? p[(int64_t)row * k + f] : (double)sp[l * row + f];
-        v = halo[t] + beta * old;
+      for (int f = tid - side * (THREADS / 2); f < row; f += THREADS / 2) {
+        const double v = next_direction(di[f], ri[f], beta, pi[f]);
+        pi[f] = v;
+        to[f] = (T)v;
       }
-      if (MIXED) p[(int64_t)row * k + f] = v;
-      sp[l * row + f] = (T)v;
+    } else {
+      const double* z = halo + side * row;
+#pragma unroll 1
+      for (int f = tid - side * (THREADS / 2); f < row; f += THREADS / 2) to[f] = fma(beta, to[f], z[f]);
     }
   }
 
@@ -676,7 +692,18 @@ struct Solver {
       const int64_t ge = d.eoff + (e - l * nxy) + (int64_t)nxy * wrap_layer(k0 - below + l);
       if (resident) info[e] = (uint16_t)element_info(ge);
     }
-    if (lean) halo_direction(0.0, true);
+    if (!lean) return;
+    const int row = 3 * nxy;
+#pragma unroll 1
+    for (int t = tid; t < 2 * row; t += THREADS) {  // the first direction beside the slab
+      const int side = t >= row, f = t - side * row;
+      const int k = side ? k1 : k0 - 1;
+      const int64_t i = (int64_t)row * k + f, g = (int64_t)row * wrap_layer(k) + f;
+      const double di = dinv_in[g], v = di * b[g];
+      if (wide) const_cast<double*>(dinv)[i] = di;
+      if (MIXED) p[i] = v;
+      sp[(side ? k1 - k0 + 1 : 0) * row + f] = (T)v;
+    }
   }
 
   __device__ __forceinline__ void solve(int s) {
@@ -752,9 +779,13 @@ struct Solver {
         const double alpha = rz / pap;
         // r -= alpha Ap at up to three entries f0, f0 + step, .. of layer k (or of the slab, MIXED)
         double next;
-        auto send = [&](int k, int f, double z) {
-          if (k == k0) cl.map_shared_rank(halo, prev_rank)[row + f] = z;
-          if (k == k1 - 1) cl.map_shared_rank(halo, next_rank)[f] = z;
+        // the neighbours' copies of the slab's first and last layer
+        auto to_prev = [&]() {
+          return MIXED ? cl.map_shared_rank(r + (int64_t)row * k0, prev_rank) + prev_layers * row
+                       : cl.map_shared_rank(halo, prev_rank) + row;
+        };
+        auto to_next = [&]() {
+          return MIXED ? cl.map_shared_rank(r + (int64_t)row * k0, next_rank) - row : cl.map_shared_rank(halo, next_rank);
         };
         if constexpr (MIXED) {
           double v[2] = {0.0, 0.0};
@@ -778,11 +809,16 @@ struct Solver {
               r[own + t] = rn;
               v[0] += rn * rn;
               v[1] += z * rn;
-              if (opaque(lean)) {
-                const int l = (int)(((float)t + 0.5f) * inv_row);
-                send(k0 + l, t - l * row, z);
-              }
             }
+          }
+          if (opaque(lean) && entries > 0) {  // every thread sends what it wrote
+            double* to = to_prev();
+#pragma unroll 1
+            for (int t = tid; t < row; t += THREADS) to[t] = r[own + t];
+            to = to_next();
+            const int from = entries - row;
+#pragma unroll 1
+            for (int t = from + (tid + THREADS - from % THREADS) % THREADS; t < entries; t += THREADS) to[t - from] = r[own + t];
           }
           sums(PART_RR, v);
           rr = v[0];
@@ -807,12 +843,15 @@ struct Solver {
                 }
 #pragma unroll
                 for (int j = 0; j < 3; ++j) {
-                  const double rn = rv[j] - alpha * av[j], z = di[j] * rn;
+                  const double rn = rv[j] - alpha * av[j], z = __dmul_rn(di[j], rn);
                   rs += rn * rn;
                   rzs += rn * z;
                   if (f0 + 32 * j >= row) continue;
                   r[i + 32 * j] = rn;
-                  if (opaque(lean)) send(k, f0 + 32 * j, z);
+                  if (opaque(lean)) {
+                    if (k == k0) to_prev()[f0 + 32 * j] = z;
+                    if (k == k1 - 1) to_next()[f0 + 32 * j] = z;
+                  }
                 }
               }
             store_parts(PART_RR, u, rs, rzs);
@@ -843,7 +882,7 @@ struct Solver {
             for (int j = 0; j < 2; ++j) {
               const int t = t0 + j * THREADS;
               if (t >= entries) continue;
-              const double v = di[j] * rv[j] + beta * pv[j];
+              const double v = next_direction(di[j], rv[j], beta, pv[j]);
               x[own + t] = xv[j] + alpha * pv[j];
               p[own + t] = v;
               if (!opaque(resident)) continue;
@@ -873,7 +912,7 @@ struct Solver {
                 for (int j = 0; j < 3; ++j) {
                   if (f0 + 32 * j >= row) continue;
                   x[i + 32 * j] = xv[j] + alpha * pv[j];
-                  put_direction(k, f0 + 32 * j, i + 32 * j, di[j] * rv[j] + beta * pv[j]);
+                  put_direction(k, f0 + 32 * j, i + 32 * j, next_direction(di[j], rv[j], beta, pv[j]));
                 }
               }
           }
@@ -883,7 +922,7 @@ struct Solver {
           break;
         }
         if (lean) {
-          if (k1 > k0) halo_direction(beta, false);
+          if (k1 > k0) halo_direction(beta);
           __syncthreads();
         } else {
           barrier();  // the direction of every rank is visible before the next apply
