@@ -858,6 +858,7 @@ def auto_pcg_cluster(batch: RVEBatch) -> int:
 
 PCG_SHAPES = {0: "256 threads (FP64: 128 or 256 by the grid)", 1: "128 threads", 2: "512 threads (FP64: 256)",
               3: "256 threads (FP64: 64)"}
+PCG_KERNELS = 2  # of the launches that stored choices were measured on: what shapes mean, what they cost
 
 
 def _tuning_path() -> Path:
@@ -868,13 +869,14 @@ def _tuning_path() -> Path:
 
 
 def _edge_mix_key(batch: RVEBatch) -> str:
-    """The tuning key of a batch: precision, GPU name and the multiset of RVE divisions."""
+    """The tuning key of a batch: version of the kernels, precision, GPU name and the multiset of
+    RVE divisions."""
     mix: dict[str, int] = {}
     for m in batch.models:
         d = "x".join(str(int(v)) for v in m.divisions)
         mix[d] = mix.get(d, 0) + 1
     name = torch.cuda.get_device_name(batch.device)
-    return f"f{batch.precision}|{name}|" + ",".join(f"{k}:{mix[k]}" for k in sorted(mix))
+    return f"v{PCG_KERNELS}|f{batch.precision}|{name}|" + ",".join(f"{k}:{mix[k]}" for k in sorted(mix))
 
 
 def tune_pcg_cluster(batch: RVEBatch, update_settings: MaterialUpdateSettings, candidates=(1, 2, 4, 8),
@@ -883,7 +885,7 @@ def tune_pcg_cluster(batch: RVEBatch, update_settings: MaterialUpdateSettings, c
     committed fluctuation) for every admissible cluster size x launch shape (threads per
     CTA, ``PCG_SHAPES``; shapes apply to cluster sizes above 1) and keep
     the fastest.  The solves write only work vectors; the batch's state is unchanged.
-    With ``persist`` the choice is stored per edge mix (precision, GPU, RVE divisions) in
+    With ``persist`` the choice is stored per edge mix (kernels, precision, GPU, RVE divisions) in
     a JSON file (``$CIB_TUNING_CACHE``, else ``~/.cache/cib200/pcg_tuning.json``) and a
     later call for the same mix takes it from there without timing.  Returns
     {"cluster": c, "shape": s, "ms": {"c/s": milliseconds}, "cached": bool, "key": key}."""
@@ -909,6 +911,9 @@ def tune_pcg_cluster(batch: RVEBatch, update_settings: MaterialUpdateSettings, c
             continue
         for shape in (shapes if c > 1 else (0,)):
             batch.cluster, batch.pcg_shape = c, shape
+            if shape == 3 and batch.precision == 32 and f"{c}/0" in timings:  # the launch of shape 0
+                timings[f"{c}/3"] = timings[f"{c}/0"]
+                continue
             for rep in range(2):  # the first run also sets the launch attributes
                 start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
                 start.record()

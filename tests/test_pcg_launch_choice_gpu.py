@@ -1,7 +1,10 @@
 """GPU tests of the choice of the RVE PCG's launch: one CTA per system is the same solve whatever
-the shape bits, and the number of systems, which decides over the CTAs of each, changes none."""
+the shape bits, the number of systems, which decides over the CTAs of each, changes none, and a
+stored choice counts for the kernels that it was measured on."""
 
 from __future__ import annotations
+
+import json
 
 import numpy as np
 import pytest
@@ -9,6 +12,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
+from concrete_impact_b200 import rve as R  # noqa: E402
 from concrete_impact_b200.rve import LinearSolverOptions, RVEBatch  # noqa: E402
 from concrete_impact_b200.rve_builders import build_two_phase_sphere_rve, config0_materials, default_newton  # noqa: E402
 from test_rve_pcg_shapes_gpu import SETTINGS, _batch, _solve  # noqa: E402
@@ -50,3 +54,19 @@ def test_solve_does_not_depend_on_the_systems_beside_it(systems: int, precision:
     together = solve(list(range(systems)), cluster)
     for i in (0, systems // 2, systems - 1):
         assert torch.equal(solve([i], cluster if precision == 32 else 1)[0], together[i]), i
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+def test_stored_choice_of_other_kernels_is_measured_again(tmp_path, monkeypatch, precision) -> None:
+    path = tmp_path / "tuning.json"
+    monkeypatch.setenv("CIB_TUNING_CACHE", str(path))
+    batch, _ = _batch((5, 4, 4), precision, 2)
+    # the key without a version, as it was stored for kernels whose shapes meant other launches
+    old = f"f{precision}|{torch.cuda.get_device_name(batch.device)}|5x4x4:2"
+    path.write_text(json.dumps({old: {"cluster": 4, "shape": 3, "ms": {}}}))
+    first = R.tune_pcg_cluster(batch, SETTINGS)
+    assert not first["cached"] and first["key"] != old
+    assert set(first["ms"]) == {"1/0"} | {f"{c}/{s}" for c in (2, 4) for s in range(4)}
+    assert old in json.loads(path.read_text())  # other entries stay
+    again = R.tune_pcg_cluster(batch, SETTINGS)
+    assert again["cached"] and (again["cluster"], again["shape"]) == (first["cluster"], first["shape"])
