@@ -453,8 +453,9 @@ __host__ __device__ inline size_t tile_smem(int layers) {
 // reciprocal estimate, one Newton step, and one correction of the quotient by its exact
 // remainder.  They are straight-line code, so the units of a thread overlap where a division's
 // own branch serialises them.  For |z| <= 69, where d stays below 2^100 and its reciprocal a
-// normal number (the caller divides elsewhere): there all floats z were compared with the
-// divisions and gave the same q and h (a zero h may differ in its sign).
+// normal number (the caller divides elsewhere); a zero h may differ from the division's in its
+// sign.  tests/test_energy_quotients_gpu.py compares silu and silu' with the divisions over every
+// 499th float from 1e-30 to 120 of both signs: the same bits.
 __device__ __noinline__ float2 silu_general(float z) { return make_float2(silu(z), silu_prime(z)); }
 
 __device__ __forceinline__ float silu_fast(float z, float d, float& q) {
