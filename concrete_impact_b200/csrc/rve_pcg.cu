@@ -53,16 +53,6 @@ enum { PART_FIRST = 0, PART_REST, PART_RR, PART_RZ, PART_XX, PART_ZERO, PART_COU
 
 // 4 consecutive tangent values (the points of one x half), as 16-byte loads when VEC.
 template <bool VEC>
-__device__ __forceinline__ void load4(const float* p, float (&v)[4]) {
-  if (VEC) {
-    const float4 t = __ldg(reinterpret_cast<const float4*>(p));
-    v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
-  } else {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = __ldg(p + k);
-  }
-}
-template <bool VEC>
 __device__ __forceinline__ void load4(const double* p, double (&v)[4]) {
   if (VEC) {
     const double2 s = __ldg(reinterpret_cast<const double2*>(p)), t = __ldg(reinterpret_cast<const double2*>(p) + 1);
@@ -75,25 +65,25 @@ __device__ __forceinline__ void load4(const double* p, double (&v)[4]) {
 
 // tau = C eps at the points of one element: C = K 1(x)1 + f P + c n(x)n at a viscoplastic
 // point (its flag set), f = 2G, c = 0 at an elastic one.
-template <typename T, bool VEC>
+template <bool VEC>
 struct TangentPoint {
-  const T* __restrict__ tparam;  // component 0 of the element's first point
+  const double* __restrict__ tparam;  // component 0 of the element's first point
   int64_t stride;   // between components
   uint32_t flags;   // bit q: point q is viscoplastic
-  T K, two_g;
-  T n[6][4], f[4], c[4];
+  double K, two_g;
+  double n[6][4], f[4], c[4];
 
   __device__ __forceinline__ void half(int h) {
     const uint32_t four = (flags >> (4 * h)) & 15u;
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
 #pragma unroll
-      for (int k = 0; k < 6; ++k) n[k][t] = (T)0;
+      for (int k = 0; k < 6; ++k) n[k][t] = 0.0;
       f[t] = two_g;
-      c[t] = (T)0;
+      c[t] = 0.0;
     }
     if (four) {
-      const T* p = tparam + 4 * h;
+      const double* p = tparam + 4 * h;
 #pragma unroll
       for (int k = 0; k < 6; ++k) load4<VEC>(p + k * stride, n[k]);
       load4<VEC>(p + 6 * stride, f);
@@ -103,19 +93,19 @@ struct TangentPoint {
         for (int t = 0; t < 4; ++t)
           if (!((four >> t) & 1u)) {
 #pragma unroll
-            for (int k = 0; k < 6; ++k) n[k][t] = (T)0;
+            for (int k = 0; k < 6; ++k) n[k][t] = 0.0;
             f[t] = two_g;
-            c[t] = (T)0;
+            c[t] = 0.0;
           }
     }
   }
 
-  __device__ __forceinline__ void operator()(int t, const T (&e)[6], T (&s)[6]) const {
-    const T tr = e[0] + e[1] + e[2];
-    const T ne = n[0][t] * e[0] + n[1][t] * e[1] + n[2][t] * e[2] + n[3][t] * e[3] + n[4][t] * e[4] + n[5][t] * e[5];
-    const T cne = c[t] * ne;
-    const T vol = K * tr - f[t] * tr * (T)(1.0 / 3.0);
-    const T hf = (T)0.5 * f[t];
+  __device__ __forceinline__ void operator()(int t, const double (&e)[6], double (&s)[6]) const {
+    const double tr = e[0] + e[1] + e[2];
+    const double ne = n[0][t] * e[0] + n[1][t] * e[1] + n[2][t] * e[2] + n[3][t] * e[3] + n[4][t] * e[4] + n[5][t] * e[5];
+    const double cne = c[t] * ne;
+    const double vol = K * tr - f[t] * tr * (1.0 / 3.0);
+    const double hf = 0.5 * f[t];
 #pragma unroll
     for (int k = 0; k < 3; ++k) s[k] = vol + f[t] * e[k] + cne * n[k][t];
 #pragma unroll
@@ -489,7 +479,7 @@ struct Solver {
         const int in = (aa & 1) ? ((aa & 2) ? n11 : n10) : ((aa & 2) ? n01 : n00);
         return ((aa & 4) ? top : bot)[in + dd];
       };
-      std::conditional_t<MIXED, TangentPair<VEC>, TangentPoint<T, VEC>> pt;
+      std::conditional_t<MIXED, TangentPair<VEC>, TangentPoint<VEC>> pt;
       const uint32_t w = info[first * nxy + e];
       pt.flags = w & 255u;
       pt.stride = a.ngp;

@@ -33,6 +33,7 @@ from .assembly import assemble_hex8_material_response_cached, build_hex8_materia
 from .materials import MaterialState, _Io
 
 CSR_PCG_WORK_DOUBLES = 3 * 1024 + 8  # CIB_CSR_PCG_WORK_DOUBLES
+CSR_PCG_BLOCK_WORK_DOUBLES = (12, 24576)  # CIB_CSR_PCG_BLOCK_WORK_DOUBLES(n): per row, and beside
 
 
 class _DeviceCSR:
@@ -100,7 +101,8 @@ class _ReducedSystem:
             rows = [self.solve(lib, b) for b in rhs]
             return torch.stack([x for x, _, _, _ in rows]), [status for _, status, _, _ in rows]
         if self.block_work is None:
-            self.block_work = torch.empty(12 * self.n + 24576, dtype=torch.float64, device=self.device)
+            per_row, beside = CSR_PCG_BLOCK_WORK_DOUBLES
+            self.block_work = torch.empty(per_row * self.n + beside, dtype=torch.float64, device=self.device)
         x = torch.empty((6, self.n), dtype=torch.float64, device=self.device)
         status, iterations, rel = (ctypes.c_int32 * 6)(), (ctypes.c_int32 * 6)(), (ctypes.c_double * 6)()
         _native.check(lib.cib_csr_pcg_block(self.n, self.indptr.data_ptr(), self.indices.data_ptr(),

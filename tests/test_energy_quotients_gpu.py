@@ -34,7 +34,7 @@ def _model(width: int) -> EnergyDissipationRVERNO:
 
 
 def test_silu_and_its_derivative_have_the_bits_of_the_divisions() -> None:
-    # every 499th float from 1e-30 to 120 of both signs (2^23 x 113 / 499 = 1.9 million each),
+    # every 499th float from 1e-30 to 120 of both signs (2^23 x 107 / 499 = 1.8 million each),
     # and 2^18 floats on either side of the range's end
     lo, hi = (int(np.float32(v).view(np.int32)) for v in (1.0e-30, 120.0))
     edge = int(np.float32(69.0).view(np.int32))

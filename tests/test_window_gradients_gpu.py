@@ -28,7 +28,7 @@ def test_every_slice_of_a_split_product_is_written(m: int, k: int, splits: int) 
 
 
 @pytest.mark.parametrize("paths, steps, hidden", [(300, 50, 128), (464, 50, 128), (768, 25, 128), (1000, 25, 128),
-                                                  (1024, 50, 128), (512, 50, 128), (300, 50, 64), (7, 1, 128)])  # fmt: skip
+                                                  (1024, 50, 128), (512, 50, 128), (300, 50, 64), (50, 6, 16), (7, 1, 128)])  # fmt: skip
 def test_window_gradients_are_the_products_of_their_operands(paths: int, steps: int, hidden: int) -> None:
     """All four layers against float64 products of the window's own bf16 operands, twice in a row
     (the second time over what the first left in the work buffers).  A slice of at most 1,024
