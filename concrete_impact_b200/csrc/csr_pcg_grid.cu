@@ -421,7 +421,9 @@ __global__ void __launch_bounds__(Shape<NV>::THREADS, 1) csr_pcg_grid_kernel(con
       else if (!(pq > 0.0) || !isfinite(pq))
         status = 2;
       if (status == 0) {
-        const double inverse = 1.0 / pq, alpha = rz * inverse;
+        const double inverse = 1.0 / pq;
+        const bool tiny = !isfinite(inverse);  // a right-hand side near the end of the range
+        const double alpha = tiny ? rz / pq : rz * inverse;
 #pragma unroll 1
         for (int i = mine; i < nr; i += STEP) {
           const int k = v * g.rows_per + i;
@@ -431,7 +433,8 @@ __global__ void __launch_bounds__(Shape<NV>::THREADS, 1) csr_pcg_grid_kernel(con
           x[k] = fma(alpha, p[v * used + own + i], x[k]);
         }
         // the next r.z over this one; rounding can leave nothing of it
-        beta = fmax(fma(fma(alpha, sums[QQ * NV + v], -2.0 * sums[ZQ * NV + v]), inverse, 1.0), 0.0);
+        const double change = fma(alpha, sums[QQ * NV + v], -2.0 * sums[ZQ * NV + v]);
+        beta = fmax(tiny ? 1.0 + change / pq : fma(change, inverse, 1.0), 0.0);
       }
     }
     __syncthreads();  // p of the own rows has been read
