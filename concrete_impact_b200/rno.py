@@ -534,13 +534,16 @@ class RNOSurrogate:
         device, strain and rate FP32 or FP64, the latent state FP32, all of them outside the two
         ``states`` (2, M, 6) that the step writes point by point (the latent state may be one of
         the two).  Anything else goes through torch."""
-        wide, begin, size = (torch.float32, torch.float64), states.data_ptr(), states.numel() * 4
-        for t, kinds in ((strain, wide), (rate, wide), (z, wide[:1])):
-            if not (t.shape == states.shape[1:] and t.device == states.device and t.is_contiguous() and t.dtype in kinds
-                    and not t.requires_grad):  # fmt: skip
+        shape, device, begin = states.shape[1:], states.get_device(), states.data_ptr()
+        size = 24 * shape[0]  # bytes of a state, half of those of an FP64 input
+        for t in (strain, rate, z):
+            if t.shape != shape or t.get_device() != device or t.requires_grad or not t.is_contiguous():
                 return False
             at = t.data_ptr() - begin
-            if -t.numel() * t.element_size() < at < size and not (t is z and at in (0, size // 2)):
+            if t.dtype is torch.float64:
+                if t is z or -2 * size < at < 2 * size:
+                    return False
+            elif t.dtype is not torch.float32 or -size < at < 2 * size and not (t is z and at in (0, size)):
                 return False
         return size > 0
 
