@@ -79,7 +79,8 @@ class MaterialAssemblyCache:
         both, home = self._host["csr"]
         if stream != home:  # it may be freed on the stream that it came from
             both.record_stream(torch.cuda.current_stream(both.device))
-        return torch.split(both.clone(), (self.csr_indptr.size, self.csr_indices.size))
+        own, rows = both.clone(), self.csr_indptr.size
+        return own[:rows], own[rows:]
 
     @property
     def jacobian_weights(self) -> np.ndarray:
