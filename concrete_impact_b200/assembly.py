@@ -71,7 +71,7 @@ class MaterialAssemblyCache:
     @property
     def csr_pattern(self) -> tuple[torch.Tensor, torch.Tensor]:
         """csr_indptr and csr_indices on the device, for one tangent to own: a copy on the device
-        (32 x 8 x 8 elements: 9 us of a call's 205) of what is uploaded once."""
+        (32 x 8 x 8 elements: 3 to 8 us of a call's 205) of what is uploaded once."""
         stream = _native.stream_ptr()
         if "csr" not in self._host:
             both = np.concatenate([self.csr_indptr, self.csr_indices])

@@ -166,8 +166,8 @@ __device__ __forceinline__ BoxGrad<T> box_grad(double hx, double hy, double hz) 
 // (x[m], x[m + 1]) at an upper one, dN_a / dz is the same at both.  The signs (plus where the
 // node's bit is set) go to the displacements; in the divergence a common sign is taken out, so
 // that one factor at most is negative.  Rounding is symmetric: the results are those of the
-// signed gradients.  Bound by issue slots between the solve's barriers: 96 RVEs of 24^3, a whole
-// batch step 73 -> 58 ms against one point to an instruction.
+// signed gradients.  Bound by issue slots between the solve's barriers: a batch step of 96 RVEs of
+// edges 8 to 24 73 -> 58 ms against one point to an instruction.
 template <typename Node, typename Point, typename Out>
 __device__ __forceinline__ void box_element_points(const BoxGrad<float>& g, float w, const Node& node, Point& point,
                                                    const Out& out) {

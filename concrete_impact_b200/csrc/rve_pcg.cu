@@ -24,12 +24,13 @@
 // block and rank in the order of a plain strided loop, which fixes the result for a given C
 // and block size.
 //
-// What bounds it: latency.  An 8^3 FP64 iteration over 8 CTAs is 14,000 cycles (7.6 us; one
+// What bounds it: latency.  An 8^3 FP64 iteration over 8 CTAs is 14,000 cycles (7.5 us; one
 // thread per Gauss point: 36.5 us on one CTA, 9.1 on eight): 4,500 element apply, 1,900 gather,
 // 3,200 barriers, 2,300 partial sums, 3,100 vector updates.  Full grids overlap two or four
-// CTAs per SM: 1,152 8^3 systems 9.9 ms (23.9), 512 in FP32 3.5 ms (6.0), 96 uneven FP32
-// systems over 8 CTAs 9.2 ms (14.5); in brackets a thread per Gauss point with the vectors in
-// L2.
+// CTAs per SM: 1,152 8^3 systems 9.9 ms (24.0), 512 in FP32 2.8 ms (6.0), 96 uneven FP32
+// systems over 8 CTAs 7.8 ms (14.7); in brackets a thread per Gauss point with the vectors in
+// L2.  Below some 64 elements a thread per element leaves too few threads: 8 x 8 x 1 takes
+// 5.9 us an iteration (5.2), 2 x 2 x 2 in FP32 5.6 (4.9).
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
