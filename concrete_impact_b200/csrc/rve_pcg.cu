@@ -1063,7 +1063,7 @@ int resident_clusters(int C) {
   int n = 0;
   if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) != cudaSuccess) {
     cudaGetLastError();
-    n = 0;
+    return 0;
   }
   kept[dev][C].store(1 + n);
   return n;
