@@ -227,7 +227,9 @@ struct Solver {
   int prev_rank, prev_layers, next_rank;  // owners of the layers below k0 and from k1 on
   bool wraps;     // one rank owns every layer (the same on every rank: it decides barriers)
   bool lean, onchip, resident;  // resident: sp holds the slab's direction during the solve
-  bool wide;      // MIXED, lean: dinv of the layers beside the slab is on chip as well
+  bool wide;      // MIXED, lean: dinv of the layers beside the slab is on chip as well (during the solve
+                  // in a partial sum that MIXED does not use: FP32 has no register left, 24^3 over 8
+                  // CTAs 8.31 ms, 8.48 with the flag in one)
   bool sends;     // the first node layer's direction goes to the rank below (resident, not lean)
   int kb;         // element layers per step
   int below;      // 1 when sp, ye and info begin at layer k0 - 1 (lean), else 0
@@ -656,7 +658,7 @@ struct Solver {
     T* to = sp + (side ? k1 - k0 + 1 : 0) * row;
     if constexpr (MIXED) {
       const int64_t i = (int64_t)row * k;
-      const double* di = wide ? dinv + i : dinv_in + (int64_t)row * wrap_layer(k);
+      const double* di = parts[PART_ZERO * WARPS] != 0.0 ? dinv + i : dinv_in + (int64_t)row * wrap_layer(k);
       const double* ri = r + i;
       double* pi = p + i;
 #pragma unroll 1
@@ -675,7 +677,8 @@ struct Solver {
   __device__ __forceinline__ void prologue() {
     const int layers = k1 - k0;
 #pragma unroll 1
-    for (int t = tid; t < PART_COUNT * (MIXED ? WARPS : octs * columns); t += THREADS) parts[t] = 0.0;
+    for (int t = tid; t < PART_COUNT * (MIXED ? WARPS : octs * columns); t += THREADS)
+      parts[t] = MIXED && wide && t == PART_ZERO * WARPS ? 1.0 : 0.0;
     if (layers == 0) return;
 #pragma unroll 1
     for (int e = tid; e < (layers + below) * nxy; e += THREADS) {
